@@ -1,0 +1,92 @@
+"""The octant copies of the nodes (ONode) against the node-by-node kernel.
+
+The while-while kernels walk per-octant copies whose children are in push
+order and whose planes are near/far; the step-scheduled kernel (tuning
+kernel 0) walks the nodes themselves.  Both must give the same bits for every
+ray and every box an upload may hold: directions with zero, negative zero,
+infinite and NaN components, boxes out of order, with NaN or infinite planes,
+empty children, one key or several, finite and infinite reach.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+OUT = ("prim", "t", "u", "v", "w")
+
+
+def _rays(n, seed):
+    from vermeer_gb300 import scenes
+    r = scenes.incoherent_rays(n, seed)
+    d = r[:, 3:6]
+    d[0::16, 0] = 0.0
+    d[1::16, 1] = -0.0
+    d[2::16, 2] = 0.0
+    d[3::16, :2] = 0.0
+    d[4::16] = (0.0, -1.0, -0.0)
+    d[5::64, 0] = np.inf
+    d[6::64, 1] = np.nan
+    d[7::64, 2] = 1e-42
+    r[8::64, 0] = np.inf
+    r[9::64, 3:6] *= 1e20
+    r[10::16, 6] = 0.3
+    r[11::64, 6] = np.nan
+    r[12::64, 6] = -1.0
+    r[:, 7] = scenes.uniform(seed, n, 77).astype(np.float32)
+    r[13::16, 7] = 0.0
+    r[14::16, 7] = 1.0
+    return r
+
+
+def _spoil(boxes, kind):
+    b = boxes.reshape(-1, 24)
+    if kind == "swapped":
+        b[::3, [0, 12]] = b[::3, [12, 0]]
+        b[1::5, [6, 18]] = b[1::5, [18, 6]]
+    elif kind == "nan":
+        b[::4, 3] = np.nan
+        b[1::4, 14] = np.nan
+        b[2::7] = np.nan
+    elif kind == "inf":
+        b[::3, 0:4] = -np.inf
+        b[::3, 12:16] = np.inf
+
+
+@pytest.mark.parametrize("kind", ["clean", "swapped", "nan", "inf"])
+@pytest.mark.parametrize("keys", [1, 2, 3])
+@pytest.mark.parametrize("tris", [1, 3, 17, 1500])
+def test_octant_copies_equal_the_nodes(ctx, kind, keys, tris):
+    from vermeer_gb300 import scenes
+    v, ip = scenes.triangle_soup(tris, 11, edge=0.2 if tris < 100 else 0.06)
+    if keys > 1:
+        vs = [v + np.float32(0.1 * k) * scenes.unit_sphere(5 + k, v.shape[0], 3).astype(np.float32)
+              for k in range(keys)]
+        v = np.concatenate(vs).astype(np.float32)
+    g = ctx.mesh_build(v, ip, keys=keys, motion_mode=1)
+    if kind != "clean":
+        e = ctx.mesh_export(g)
+        if keys == 1:
+            nodes = e["nodes"].copy()
+            boxes = np.ascontiguousarray(nodes["boxes"])
+            _spoil(boxes, kind)
+            nodes["boxes"] = boxes
+            g = ctx.mesh_upload(v, e["idxp"], e["accel_idx"], nodes=nodes, bounds=e["bounds"])
+        else:
+            boxes = e["mboxes"].copy()
+            _spoil(boxes, kind)
+            g = ctx.mesh_upload(v, e["idxp"], e["accel_idx"], mnodes=e["mnodes"], mboxes=boxes, bounds=e["bounds"],
+                                keys=keys, motion_mode=1)
+    rays = _rays(4099, 3)
+    try:
+        for shadow in (False, True):
+            got = {}
+            for k in (0, 13, 45):
+                ctx.set_tuning(kernel=k)
+                got[k] = ctx.trace_mesh(g, rays, shadow=shadow)
+            assert (got[0]["prim"] >= 0).any() or kind == "nan" or tris < 100
+            for k in (13, 45):
+                for o in OUT:
+                    a, b = got[k][o], got[0][o]
+                    a, b = (x.view(np.uint32) if x.dtype == np.float32 else x for x in (a, b))
+                    assert np.array_equal(a, b), (o, k, shadow)
+    finally:
+        ctx.set_tuning()

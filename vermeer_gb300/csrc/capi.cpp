@@ -122,6 +122,22 @@ void fill_xf(const MeshRec& rec, DMesh& d) {
   d.xf_keys = keyed ? rec.dxkeys.as<vmr::anim::Decomp>() : nullptr;
 }
 
+// The octant copies of n nodes.  They only save work: without the memory for
+// them the traces walk the nodes themselves.
+cudaError_t octant_nodes(vmr_ctx* ctx, const DevBuf& nodes, uint32_t n, DevBuf& buf, const vmr::ONode*& out) {
+  out = nullptr;
+  if (n == 0) return cudaSuccess;
+  cudaError_t e = buf.ensure((size_t)8 * n * sizeof(vmr::ONode));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  if (e != cudaSuccess) return e;
+  e = (cudaError_t)vmr::launch_octant_nodes(nodes.as<GNode>(), n, buf.as<vmr::ONode>(), ctx->stream);
+  if (e == cudaSuccess) out = buf.as<vmr::ONode>();
+  return e;
+}
+
 // Host accelerator -> device arrays (layout in device.h).  tris_ready: the
 // device builder already wrote the static triangle table into rec.tris.
 int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
@@ -145,6 +161,8 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
       VMR_CUDA(ctx, upload(ctx, rec.tris, tris));
     }
     d.nodes = rec.nodes.as<GNode>();
+    d.n_nodes = (uint32_t)m.nodes.size();
+    VMR_CUDA(ctx, octant_nodes(ctx, rec.nodes, d.n_nodes, rec.onodes, d.onodes));
     d.tris = rec.tris.p;
     d.iter_cap = 4u * (uint32_t)m.nodes.size() + 2u;
   } else {
@@ -168,6 +186,27 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
     VMR_CUDA(ctx, upload(ctx, rec.mboxes, m.mboxes));
     VMR_CUDA(ctx, upload(ctx, rec.mtris, tris));
     VMR_CUDA(ctx, upload(ctx, rec.elem, elem));
+    int bad = 0;
+    const uint32_t nm = (uint32_t)m.mnodes.size();
+    // obase + keys * n_nodes stays in 32 bits (the kernels' index)
+    if ((uint64_t)8 * m.keys * nm < 0xfffffffeull) {
+      const size_t ob = (size_t)8 * m.keys * nm * sizeof(vmr::ONode);
+      const cudaError_t e = rec.onodes.ensure(ob + 16);
+      if (e == cudaSuccess) {
+        int* flag = reinterpret_cast<int*>(rec.onodes.as<char>() + ob);
+        const int le = vmr::launch_octant_mnodes(rec.mnodes.as<MNode>(), rec.mboxes.p, m.keys, nm,
+                                                 rec.onodes.as<vmr::ONode>(), flag, ctx->stream);
+        if (le != 0) return cuda_fail(ctx, (cudaError_t)le, "octant nodes launch");
+        VMR_CUDA(ctx, cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (!bad) d.onodes = rec.onodes.as<vmr::ONode>();
+      } else if (e == cudaErrorMemoryAllocation) {  // the traces walk mnodes
+        cudaGetLastError();
+      } else {
+        return cuda_fail(ctx, e, "octant nodes");
+      }
+    }
+    d.n_nodes = nm;
     d.mnodes = rec.mnodes.as<MNode>();
     d.mboxes = rec.mboxes.p;
     d.mtris = rec.mtris.p;

@@ -39,7 +39,7 @@ struct DevBuf {
 
 struct MeshRec {
   HostMesh host;
-  DevBuf nodes, tris, mnodes, mboxes, mtris, elem;
+  DevBuf nodes, onodes, tris, mnodes, mboxes, mtris, elem;
   DMesh dmesh{};
   float bounds6[6];
   // shading (render.cu): PolyMesh.Shader, shader index and normals per

@@ -41,6 +41,24 @@ struct alignas(128) GNode {
 };
 static_assert(sizeof(GNode) == 128, "GNode must be 128 bytes");
 
+// A static node as the rays of one direction octant read it (o = the sign
+// bits of D): the children in push order (slot 0 pushed first, so slot 3 is
+// visited first), and per child the near and far box planes of that octant
+// instead of min and max, so a visit needs neither the min/max of each plane
+// pair nor the rank arithmetic of the push.  A mesh holds one such array per
+// octant (o * n_nodes + node): 8 x 128 B per node, about the size of the
+// triangle table.  An absent child's planes are never hit (near +inf, far
+// -inf along D).  A motion mesh holds the same per key ((o * keys + key) *
+// n_nodes + node): the near planes of two keys lerp to the near plane at the
+// ray's time, as the boxes of every key are ordered; its absent children are
+// told by their code.
+struct alignas(128) ONode {
+  float slot[4][6];     // near x, near y, far x, far y, near z, far z
+  int32_t child[4];
+  uint32_t pad[4];
+};
+static_assert(sizeof(ONode) == 128, "ONode must be 128 bytes");
+
 struct alignas(32) MNode {
   int32_t child[4];
   uint32_t axes;
@@ -52,6 +70,9 @@ static_assert(sizeof(MNode) == 32, "MNode must be 32 bytes");
 // One mesh as the kernels see it.
 struct DMesh {
   const GNode* nodes;       // static
+  const ONode* onodes;      // [8][keys][n_nodes]; null: the kernels walk nodes / mnodes
+  uint32_t n_nodes;
+  uint32_t pad0;
   const void* tris;         // float4[3*n_tris] (static)
   const MNode* mnodes;      // motion
   const void* mboxes;       // float4[keys][n_mnodes][6]
@@ -186,6 +207,13 @@ int launch_ray_sort(const RaySoA& rays, uint64_t n, const float bounds[6], int b
                     uint32_t* order, const RaySoA& sorted_out, void* stream,
                     const unsigned long long* n_dev = nullptr);
 int launch_trace_scene(const DTop& top, const TraceLaunch& l);
+// out[8][n]: the octant copies of n nodes (traverse.cu).
+int launch_octant_nodes(const GNode* nodes, uint32_t n, ONode* out, void* stream);
+// out[8][keys][n] of n motion nodes; *bad is set when a box has its planes out
+// of order or a NaN, where lerped near and far planes would not be the lerped
+// boxes' (such a mesh keeps to its mnodes).
+int launch_octant_mnodes(const MNode* nodes, const void* mboxes, uint32_t keys, uint32_t n, ONode* out, int* bad,
+                         void* stream);
 int device_sm_count();
 
 // One job of a batched trace (vmr_trace_jobs): its rays and hits (device

@@ -37,6 +37,9 @@ namespace vmr {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
+// A ray's octant copy (k_trace_mesh_ww), or one of: no copies (the nodes, plain
+// slab test), and the nodes with the operand order a NaN needs.
+constexpr uint32_t kNodesPlain = 0xfffffffeu, kNodesExact = 0xffffffffu;
 
 __device__ __forceinline__ float pick3(float x, float y, float z, int k) {
   return k == 0 ? x : (k == 1 ? y : z);
@@ -842,6 +845,17 @@ __global__ void k_jobs_scatter(const JobDesc* jobs, uint32_t n_jobs, uint64_t n,
 // with one warp-aggregated atomic (ballot of idle lanes, leader adds the
 // count, lanes take base + their rank among the idle lanes), which keeps the
 // warp full until the ray pool runs dry.
+//
+// What bounds it: load latency and the L1 data pipe (about 75% of its
+// wavefronts; a visit costs one per lane and load instruction), then issue.
+// The octant copies exist to cut the work around those loads: push order and
+// near/far planes come with the node, two axes share an instruction, and a
+// step's pops follow its visit instead of taking steps of their own (of the
+// lanes of a step a quarter found a leaf and 8% popped a culled entry).
+// 4,194,304 incoherent rays on 1,048,576 triangles: 5.51 -> 4.08 G warp
+// instructions, 19.6 -> 22.9 lanes active, whole call 6.94 -> 6.56 ms; 300,007
+// coherent shadow rays on 200,003 triangles 0.61 -> 0.56 ms; 262,147 rays on
+// 100,000 moving triangles 1.43 -> 1.35 ms.
 
 // 32 bytes of read-only global memory (32-byte aligned) as two float4, in
 // one 256-bit load: a node of 128 bytes takes four load instructions
@@ -894,6 +908,174 @@ __device__ __forceinline__ void fetch_mnode(const MNode* mnodes, int node, unsig
   rk = (((oct & 4u) ? meta.z : meta.y) >> ((oct & 3u) * 8u)) & 0xffu;
 }
 
+// ---- the octant walk of static nodes (ONode, device.h)
+// Two float32 operations in one instruction, each rounded as the scalar one
+// (add.rn / mul.rn .f32x2): the slab test's subtractions and products of two
+// axes at a time, and the three-operand min and max.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ void ld_u64x4(const void* p, uint64_t& a, uint64_t& b, uint64_t& c, uint64_t& d) {
+  asm("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+}
+
+// The slab test's view of a ray: the negated origin and Dinv, x and y in one
+// register pair and z twice in another.
+struct SlabRay {
+  uint64_t noxy, nozz, ixy, izz;
+};
+__device__ __forceinline__ SlabRay slab_ray(const TRay& r) {
+  return SlabRay{pack2(-r.ox, -r.oy), pack2(-r.oz, -r.oz), pack2(r.ix, r.iy), pack2(r.iz, r.iz)};
+}
+
+// The children of a visited node in push order: hit mask over the slots,
+// child codes and tNear.
+struct Slots {
+  unsigned mask;
+  int child[4];
+  float t[4];
+};
+
+// Slab test of one slot: (b - o) * Dinv per plane with b - o = b + (-o), the
+// near planes of the octant giving the reference's min of each plane pair
+// and the far planes its max (the products are monotone in b).  hit: tNear <=
+// tFar and not Tclosest < tNear (a child the reference culls when popped is
+// not pushed).
+__device__ __forceinline__ bool slot_hit(const SlabRay& s, float tclosest, uint64_t nxy, uint64_t fxy, uint64_t nfz,
+                                         float& t) {
+  const uint64_t n = mul2(add2(nxy, s.noxy), s.ixy), f = mul2(add2(fxy, s.noxy), s.ixy),
+                 z = mul2(add2(nfz, s.nozz), s.izz);
+  t = fmaxf(max3(lo2(n), hi2(n), lo2(z)), 0.0f);
+  return t <= fminf(min3(lo2(f), hi2(f), hi2(z)), tclosest);
+}
+
+__device__ __forceinline__ void visit_octant(const ONode* p, const SlabRay& s, float tclosest, Slots& o) {
+  uint64_t w[16];
+  const uint64_t* q = reinterpret_cast<const uint64_t*>(p);
+  ld_u64x4(q, w[0], w[1], w[2], w[3]);
+  ld_u64x4(q + 4, w[4], w[5], w[6], w[7]);
+  ld_u64x4(q + 8, w[8], w[9], w[10], w[11]);
+  const int4 c = __ldg(reinterpret_cast<const int4*>(p->child));
+  o.child[0] = c.x; o.child[1] = c.y; o.child[2] = c.z; o.child[3] = c.w;
+  o.mask = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (slot_hit(s, tclosest, w[3 * k], w[3 * k + 1], w[3 * k + 2], o.t[k])) o.mask |= 1u << k;
+}
+
+// A motion node's octant copies of both keys (p0, p1: the same node of the
+// two keys), the planes lerped per float: (1.0-time)*Boxes[key] +
+// time*Boxes[key2] (motionintersect.go:47-49); tm2, omt2: the weights twice.
+__device__ __forceinline__ void visit_octant_m(const ONode* p0, const ONode* p1, const SlabRay& s, uint64_t tm2,
+                                               uint64_t omt2, float tclosest, Slots& o) {
+  const uint64_t* q0 = reinterpret_cast<const uint64_t*>(p0);
+  const uint64_t* q1 = reinterpret_cast<const uint64_t*>(p1);
+  uint64_t w[12];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    uint64_t a[4], c[4];
+    ld_u64x4(q0 + 4 * k, a[0], a[1], a[2], a[3]);
+    ld_u64x4(q1 + 4 * k, c[0], c[1], c[2], c[3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[4 * k + j] = add2(mul2(omt2, a[j]), mul2(tm2, c[j]));
+  }
+  const int4 c = __ldg(reinterpret_cast<const int4*>(p0->child));
+  o.child[0] = c.x; o.child[1] = c.y; o.child[2] = c.z; o.child[3] = c.w;
+  o.mask = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (slot_hit(s, tclosest, w[3 * k], w[3 * k + 1], w[3 * k + 2], o.t[k]) && o.child[k] != kEmptyChild)
+      o.mask |= 1u << k;
+}
+
+__global__ void k_octant_mnodes(const MNode* __restrict__ nodes, const float* __restrict__ boxes, uint32_t keys,
+                                uint32_t n, ONode* __restrict__ out, int* bad) {
+  const uint64_t per = (uint64_t)keys * n, total = per * 8;
+  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t o = (uint32_t)(g / per);
+    const uint64_t kn = g % per;
+    const MNode& N = nodes[kn % n];
+    const float* box = boxes + kn * 24;
+    const unsigned rk = (N.rank[o >> 2] >> (8u * (o & 3u))) & 0xffu;
+    ONode r;
+    for (int c = 0; c < 4; ++c) {
+      const unsigned slot = (rk >> (2 * c)) & 3u;
+      const int at_near[3] = {0, 1, 4}, at_far[3] = {2, 3, 5};
+      for (int a = 0; a < 3; ++a) {
+        const float mn = box[c + 4 * a], mx = box[12 + c + 4 * a];
+        const bool neg = (o >> a) & 1u;
+        if (N.child[c] != kEmptyChild && !(mn <= mx)) *bad = 1;
+        r.slot[slot][at_near[a]] = neg ? mx : mn;
+        r.slot[slot][at_far[a]] = neg ? mn : mx;
+      }
+      r.child[slot] = N.child[c];
+    }
+    for (int k = 0; k < 4; ++k) r.pad[k] = 0;
+    out[g] = r;
+  }
+}
+
+// Octant copies of the nodes.  A plane pair given in the wrong order is put in
+// order and a NaN plane takes the other's value, as the min and max of the
+// products would; a child all of whose planes are NaN is never hit.
+__global__ void k_octant_nodes(const GNode* __restrict__ nodes, uint32_t n, ONode* __restrict__ out) {
+  const uint64_t total = (uint64_t)n * 8;
+  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t o = (uint32_t)(g / n);
+    const GNode& N = nodes[g % n];
+    const unsigned rk = (N.rank[o >> 2] >> (8u * (o & 3u))) & 0xffu;
+    ONode r;
+    for (int c = 0; c < 4; ++c) {
+      const unsigned slot = (rk >> (2 * c)) & 3u;
+      bool absent = N.child[c] == kEmptyChild;
+      float lo[3], hi[3];
+      int nans = 0;
+      for (int a = 0; a < 3; ++a) {
+        const float mn = N.box[c + 4 * a], mx = N.box[12 + c + 4 * a];
+        lo[a] = fminf(mn, mx);
+        hi[a] = fmaxf(mn, mx);
+        nans += isnan(lo[a]) ? 1 : 0;
+      }
+      absent = absent || nans == 3;
+      float* d = r.slot[slot];
+      const int at_near[3] = {0, 1, 4}, at_far[3] = {2, 3, 5};
+      for (int a = 0; a < 3; ++a) {
+        const bool neg = (o >> a) & 1u;
+        const float inf = __int_as_float(0x7f800000);
+        const float l = absent ? inf : lo[a], h = absent ? -inf : hi[a];
+        // absent: near +inf and far -inf along D, whichever way D points
+        d[at_near[a]] = absent ? (neg ? -inf : inf) : (neg ? h : l);
+        d[at_far[a]] = absent ? (neg ? inf : -inf) : (neg ? l : h);
+      }
+      r.child[slot] = N.child[c];
+    }
+    for (int k = 0; k < 4; ++k) r.pad[k] = 0;
+    out[g] = r;
+  }
+}
+
 // A traversal stack whose first SS entries per thread live in shared memory
 // (entry-major, so the 32 lanes of a warp always touch 32 different banks)
 // and the rest in local memory; SS = 0 keeps the whole stack local.
@@ -917,35 +1099,51 @@ struct SplitStack {
   }
 };
 
-// push_ranked for a SplitStack.
+// Push the hit slots in slot order; the last one is returned as the next
+// entry instead.
 template <class S>
-__device__ __forceinline__ bool push_ranked_s(S& stk, int& sp, unsigned mask, const int4& ch, const float (&tn)[4],
-                                              unsigned rk, int& next, float& nextT, int& status) {
-  if (mask == 0) return false;
-  const unsigned r0 = rk & 3u, r1 = (rk >> 2) & 3u, r2 = (rk >> 4) & 3u, r3 = (rk >> 6) & 3u;
-  const unsigned rmask = ((mask & 1u) << r0) | (((mask >> 1) & 1u) << r1) | (((mask >> 2) & 1u) << r2) |
-                         (((mask >> 3) & 1u) << r3);
-  const unsigned rtop = 31u - __clz(rmask);
-  const int npush = __popc(rmask) - 1;
-  if (sp + npush > kStackCapacity) {
+__device__ __forceinline__ bool push_slots(S& stk, int& sp, const Slots& o, int& next, int& status) {
+  const unsigned m = o.mask;
+  if (m == 0) return false;
+  if (sp + __popc(m) - 1 > kStackCapacity) {
     status = kStatusStackOverflow;
     return false;
   }
-  const unsigned rr[4] = {r0, r1, r2, r3};
-  const int cv[4] = {ch.x, ch.y, ch.z, ch.w};
+  next = (m & 8u) ? o.child[3] : ((m & 4u) ? o.child[2] : ((m & 2u) ? o.child[1] : o.child[0]));
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    if (mask & (1u << c)) {
-      if (rr[c] == rtop) {
-        next = cv[c];
-        nextT = tn[c];
-      } else {
-        stk.set(sp + __popc(rmask & ((1u << rr[c]) - 1u)), cv[c], tn[c]);
-      }
+  for (int k = 0; k < 3; ++k)
+    if ((m & (1u << k)) && (m >> (k + 1)) != 0u) {
+      stk.set(sp, o.child[k], o.t[k]);
+      ++sp;
     }
-  }
-  sp += npush;
   return true;
+}
+
+// The visit of the node itself (b: its boxes, at the ray's time for a motion
+// node): meshes without octant copies, and (exact) rays whose slab test can
+// meet a NaN, with the reference's MINPS/MAXPS operand order.  The children to
+// push go to out in push order; returns their number.
+__device__ __forceinline__ int visit_node(const float4 (&b)[6], const int4& ch, unsigned rk, const SlabRay& s,
+                                          bool exact, float tclosest, int2* out) {
+  TRay r;
+  r.ox = -lo2(s.noxy); r.oy = -hi2(s.noxy); r.oz = -lo2(s.nozz);
+  r.ix = lo2(s.ixy); r.iy = hi2(s.ixy); r.iz = lo2(s.izz);
+  float tn[4];
+  unsigned mask = exact ? box4<true>(r, b, tn) : box4<false>(r, b, tn);
+  if (ch.x == kEmptyChild || tclosest < tn[0]) mask &= ~1u;
+  if (ch.y == kEmptyChild || tclosest < tn[1]) mask &= ~2u;
+  if (ch.z == kEmptyChild || tclosest < tn[2]) mask &= ~4u;
+  if (ch.w == kEmptyChild || tclosest < tn[3]) mask &= ~8u;
+  const int cv[4] = {ch.x, ch.y, ch.z, ch.w};
+  unsigned rmask = 0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (mask & (1u << c)) rmask |= 1u << ((rk >> (2 * c)) & 3u);
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (mask & (1u << c))
+      out[__popc(rmask & ((1u << ((rk >> (2 * c)) & 3u)) - 1u))] = make_int2(cv[c], __float_as_int(tn[c]));
+  return __popc(mask);
 }
 
 // Push the hit children in rank order (rank r_c = bits 2c..2c+1 of rk);
@@ -1248,9 +1446,10 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
   const unsigned lanes_below = (1u << lane) - 1u;
   TRay r;
   HitRec h{-1, -1, 0.f, 0.f, 0.f};
-  // Current entry (as if just popped); -1 = no entry left.
+  // Current entry, popped and not culled; -1 = no entry left.
   int node = -1, sp = 0;
-  float nodeT = 0.f;
+  SlabRay slab{};
+  uint32_t obase = 0;  // the ray's octant copy, kNodesPlain or kNodesExact
   uint64_t rid = 0;
   uint32_t iter = 0;
   bool alive = false, hit = false;
@@ -1258,8 +1457,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
   int status = kStatusOk;
   Counters cnt{0, 0, 0};
   float tm = 0.f, omt = 1.f;
-  const float4* bx0 = nullptr;
-  const float4* bx1 = nullptr;
+  uint32_t dkey = 0;  // motion: nodes from the ray's first key to its second (n_nodes, or 0 at a key)
   const float4* tr0 = reinterpret_cast<const float4*>(MOTION ? m.mtris : m.tris);
   const float4* tr1 = tr0;
   for (;;) {
@@ -1293,7 +1491,8 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
           h = HitRec{-1, -1, 0.f, 0.f, 0.f};
           hit = false;
           node = 0;  // the root, pushed with T = Tclosest (intersect.go:93-95)
-          nodeT = r.tclosest;
+          slab = slab_ray(r);
+          obase = r.exact ? kNodesExact : !m.onodes ? kNodesPlain : r.oct * (MOTION ? m.keys : 1u) * m.n_nodes;
           sp = 0;
           iter = 0;
           alive = true;
@@ -1310,8 +1509,8 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
               store_hit(hits, rid, r, false, h);
               alive = false;
             } else {
-              bx0 = reinterpret_cast<const float4*>(m.mboxes) + (size_t)key * m.n_mnodes * 6;
-              bx1 = reinterpret_cast<const float4*>(m.mboxes) + (size_t)key2 * m.n_mnodes * 6;
+              dkey = key2 != key ? m.n_nodes : 0u;
+              if (obase < kNodesPlain) obase += (uint32_t)key * m.n_nodes;
               tr0 = reinterpret_cast<const float4*>(m.mtris) + (size_t)key * m.n_tris * 3;
               tr1 = reinterpret_cast<const float4*>(m.mtris) + (size_t)key2 * m.n_tris * 3;
             }
@@ -1325,14 +1524,26 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
       continue;
     }
     constexpr bool kCoop = COOP;
-    bool done = false, walking = false;
+    bool done = false, walking = node >= 0;
+    // The next entry of the stack the reference does not cull when it pops
+    // it (Tclosest < T, intersect.go:106); -1: none left.
+    auto pop = [&]() {
+      for (;;) {
+        if (sp == 0) {
+          node = -1;
+          return;
+        }
+        const int2 e = stk.get(--sp);
+        node = e.x;
+        if (!(r.tclosest < __int_as_float(e.y))) return;
+      }
+    };
     if (alive) {
-      // ---- node phase: one entry per step (a cull-pop, a leaf found, or an
-      // inner-node visit) for every lane still walking.  The warp steps in
-      // lock-step; it stops when no lane walks, or when at most walk_tail
-      // lanes walk and some lane holds a leaf (the stragglers resume in the
-      // next node phase).
-      walking = node != -1;
+      // ---- node phase: one inner-node visit per step for every lane still
+      // walking; the pops (and culls) up to the next entry follow in the same
+      // step, so every walking lane of a step visits a node.  The warp
+      // stops when no lane walks, or when at most walk_tail lanes walk and some
+      // lane holds a leaf (the stragglers resume in the next node phase).
       for (;;) {
         const unsigned wmask = __ballot_sync(alive_mask, walking);
         if (wmask == 0u) break;
@@ -1347,49 +1558,48 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
           walking = false;
           continue;
         }
-        if (r.tclosest < nodeT) {  // pop-time cull (intersect.go:106)
-          if (sp == 0) {
-            node = -1;
-            walking = false;
-          } else {
-            const int2 e = stk.get(--sp);
-            node = e.x;
-            nodeT = __int_as_float(e.y);
-          }
-          continue;
-        }
-        if (node < 0) {  // a leaf: the leaf phase scans it
-          walking = false;
-          continue;
-        }
         if (COUNT) cnt.nodes++;
-        float4 b[6];
-        int4 ch;
-        unsigned rk;
-        if (MOTION) fetch_mnode(m.mnodes, node, r.oct, bx0, bx1, tm, omt, b, ch, rk);
-        else fetch_node(m, node, r.oct, b, ch, rk);
-        float tn[4];
-        unsigned mask = r.exact ? box4<true>(r, b, tn) : box4<false>(r, b, tn);
-        if (ch.x == kEmptyChild || r.tclosest < tn[0]) mask &= ~1u;
-        if (ch.y == kEmptyChild || r.tclosest < tn[1]) mask &= ~2u;
-        if (ch.z == kEmptyChild || r.tclosest < tn[2]) mask &= ~4u;
-        if (ch.w == kEmptyChild || r.tclosest < tn[3]) mask &= ~8u;
         int next = 0;
-        float nextT = 0.f;
-        if (push_ranked_s(stk, sp, mask, ch, tn, rk, next, nextT, status)) {
+        bool pushed;
+        if (obase < kNodesPlain) {
+          Slots o;
+          const ONode* on = m.onodes + (obase + (uint32_t)node);
+          if (MOTION) visit_octant_m(on, on + dkey, slab, pack2(tm, tm), pack2(omt, omt), r.tclosest, o);
+          else visit_octant(on, slab, r.tclosest, o);
+          pushed = push_slots(stk, sp, o, next, status);
+        } else {
+          float4 b[6];
+          int4 ch;
+          unsigned rk;
+          if (MOTION) {
+            const float4* bx = reinterpret_cast<const float4*>(m.mboxes);
+            const int key = (int)floorf(__fmul_rn(r.time, (float)(m.keys - 1)));
+            bx += (size_t)key * m.n_mnodes * 6;
+            fetch_mnode(m.mnodes, node, r.oct, bx, bx + (size_t)dkey * 6, tm, omt, b, ch, rk);
+          } else {
+            fetch_node(m, node, r.oct, b, ch, rk);
+          }
+          int2 e[4];
+          const int np = visit_node(b, ch, rk, slab, obase == kNodesExact, r.tclosest, e);
+          pushed = false;
+          if (sp + np - 1 > kStackCapacity) {
+            status = kStatusStackOverflow;
+          } else if (np > 0) {
+            for (int k = 0; k + 1 < np; ++k) stk.set(sp++, e[k].x, __int_as_float(e[k].y));
+            next = e[np - 1].x;
+            pushed = true;
+          }
+        }
+        if (pushed) {
           node = next;
-          nodeT = nextT;
         } else if (status != kStatusOk) {
           done = true;
           walking = false;
-        } else if (sp == 0) {
-          node = -1;
-          walking = false;
+          continue;
         } else {
-          const int2 e = stk.get(--sp);
-          node = e.x;
-          nodeT = __int_as_float(e.y);
+          pop();
         }
+        walking = node >= 0;
       }
       // ---- leaf phase: lanes whose current entry is a leaf scan it, in the
       // order the reference pops it, then pop the next entry.
@@ -1406,13 +1616,11 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
           h.w = W;
           hit = true;
         }
-        if ((ANY && idx != -1) || sp == 0) {  // shadow rays stop at the first hit leaf (intersect.go:231-236)
+        if (ANY && idx != -1) {  // shadow rays stop at the first hit leaf (intersect.go:231-236)
           done = true;
         } else {
-          const int2 e = stk.get(--sp);
-          node = e.x;
-          nodeT = __int_as_float(e.y);
-          if (PF && !MOTION && node >= 0) prefetch_l1(m.nodes + node);
+          pop();
+          if (PF && !MOTION && node >= 0 && obase < kNodesPlain) prefetch_l1(m.onodes + (obase + (uint32_t)node));
         }
       }
     }
@@ -1437,12 +1645,10 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
           h.w = W;
           hit = true;
         }
-        if ((ANY && idx != -1) || sp == 0) {
+        if (ANY && idx != -1) {
           done = true;
         } else {
-          const int2 e = stk.get(--sp);
-          node = e.x;
-          nodeT = __int_as_float(e.y);
+          pop();
         }
       }
     }
@@ -2193,6 +2399,21 @@ int launch_trace_jobs(const JobDesc* jobs, uint32_t n_jobs, uint64_t n_rays, con
   e = launch_trace_scene(top, l);
   if (e != 0) return e;
   k_jobs_scatter<<<grid, block, 0, st>>>(jobs, n_jobs, n_rays, w.hits);
+  return (int)cudaGetLastError();
+}
+
+int launch_octant_nodes(const GNode* nodes, uint32_t n, ONode* out, void* stream) {
+  const uint64_t want = ((uint64_t)n * 8 + 127) / 128, cap = (uint64_t)device_sm_count() * 32;
+  k_octant_nodes<<<(int)(want < cap ? want : cap), 128, 0, (cudaStream_t)stream>>>(nodes, n, out);
+  return (int)cudaGetLastError();
+}
+
+int launch_octant_mnodes(const MNode* nodes, const void* mboxes, uint32_t keys, uint32_t n, ONode* out, int* bad,
+                         void* stream) {
+  const uint64_t want = ((uint64_t)n * keys * 8 + 127) / 128, cap = (uint64_t)device_sm_count() * 32;
+  cudaMemsetAsync(bad, 0, sizeof(int), (cudaStream_t)stream);
+  k_octant_mnodes<<<(int)(want < cap ? want : cap), 128, 0, (cudaStream_t)stream>>>(
+      nodes, static_cast<const float*>(mboxes), keys, n, out, bad);
   return (int)cudaGetLastError();
 }
 
