@@ -90,3 +90,32 @@ def test_octant_copies_equal_the_nodes(ctx, kind, keys, tris):
                     assert np.array_equal(a, b), (o, k, shadow)
     finally:
         ctx.set_tuning()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 3039, 3041, 4255, 4257, 8513, 70001, 136193])
+def test_ray_counts_around_the_warps_share(ctx, n):
+    """A launch of few rays spreads them over its warps: one ray a warp, the
+    last warp short, two or more a warp, up to full warps (152 SMs x 7 or 5
+    blocks x 4 warps), meshes and a two-level scene of both kinds."""
+    from vermeer_gb300 import scenes
+    v, ip = scenes.triangle_soup(1500, 11, edge=0.06)
+    vm, im = scenes.motion_soup(700, 12, velocity=0.1, edge=0.06)
+    gs, gm = ctx.mesh_build(v, ip), ctx.mesh_build(vm, im, keys=2, motion_mode=1)
+    rays = _rays(n, 5)
+    scene_rays = rays[np.isfinite(rays[:, :7]).all(1)] if n > 33 else scenes.incoherent_rays(n, 5)
+    try:
+        for shadow in (False, True):
+            got = {}
+            for k in (0, 45):
+                ctx.set_tuning(kernel=k)
+                r = [ctx.trace_mesh(g, rays, shadow=shadow) for g in (gs, gm)]
+                for geoms in ([gs], [gs, gm]):
+                    ctx.scene_build(geoms)
+                    r.append(ctx.trace_scene(scene_rays, shadow=shadow))
+                got[k] = r
+            for a, b in zip(got[0], got[45]):
+                for o in OUT:
+                    x, y = (z[o].view(np.uint32) if z[o].dtype == np.float32 else z[o] for z in (a, b))
+                    assert np.array_equal(x, y), (o, shadow)
+    finally:
+        ctx.set_tuning()

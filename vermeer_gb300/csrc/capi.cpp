@@ -148,6 +148,7 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
   d.keys = m.motion() ? m.keys : 1u;
   d.lower_static = 1.19209290e-07f + m.ray_bias;  // EpsilonFloat32 + RayBias
   d.ray_bias = m.ray_bias;
+  int* bad_dev = nullptr;  // motion: set by the octant copies' kernel
   if (!m.motion()) {
     std::vector<GNode> g;
     if (!repack_nodes(m.nodes, m.n_tris, g)) return fail(ctx, VMR_ERR_INVALID, "malformed QBVH nodes");
@@ -186,7 +187,6 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
     VMR_CUDA(ctx, upload(ctx, rec.mboxes, m.mboxes));
     VMR_CUDA(ctx, upload(ctx, rec.mtris, tris));
     VMR_CUDA(ctx, upload(ctx, rec.elem, elem));
-    int bad = 0;
     const uint32_t nm = (uint32_t)m.mnodes.size();
     // obase + keys * n_nodes stays in 32 bits (the kernels' index)
     if ((uint64_t)8 * m.keys * nm < 0xfffffffeull) {
@@ -197,9 +197,7 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
         const int le = vmr::launch_octant_mnodes(rec.mnodes.as<MNode>(), rec.mboxes.p, m.keys, nm,
                                                  rec.onodes.as<vmr::ONode>(), flag, ctx->stream);
         if (le != 0) return cuda_fail(ctx, (cudaError_t)le, "octant nodes launch");
-        VMR_CUDA(ctx, cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (!bad) d.onodes = rec.onodes.as<vmr::ONode>();
+        bad_dev = flag;
       } else if (e == cudaErrorMemoryAllocation) {  // the traces walk mnodes
         cudaGetLastError();
       } else {
@@ -214,7 +212,10 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
     d.n_mnodes = (uint32_t)m.mnodes.size();
     d.iter_cap = 4u * (uint32_t)m.mnodes.size() + 2u;
   }
+  int bad = 0;
+  if (bad_dev) VMR_CUDA(ctx, cudaMemcpyAsync(&bad, bad_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (bad_dev && !bad) d.onodes = rec.onodes.as<vmr::ONode>();
   fill_xf(rec, d);
   rec.dmesh = d;
   for (int a = 0; a < 3; ++a) {

@@ -93,6 +93,14 @@ __device__ __forceinline__ void ray_setup(TRay& r) {
               r.iz != 0.0f && isfinite(r.ox) && isfinite(r.oy) && isfinite(r.oz));
 }
 
+// (Kx, Ky, Kz) of a permutation class.
+__device__ __forceinline__ void class_axes(int cls, int& kx, int& ky, int& kz) {
+  kz = cls >> 1;
+  const int a = kz == 2 ? 0 : kz + 1, b = kz == 0 ? 2 : kz - 1;  // Kz + 1 and Kz + 2 (mod 3)
+  kx = (cls & 1) ? b : a;
+  ky = (cls & 1) ? a : b;
+}
+
 // Slab test of the 4 children against boxes b[6] (intersect_amd64.s).
 // Returns the 4-bit hit mask, tNear per child in tn[].
 template <bool EXACT>
@@ -602,6 +610,22 @@ __device__ __forceinline__ void store_hit(const HitSoA& hs, uint64_t i, const TR
   if (hs.w) hs.w[i] = hit ? h.w : 0.0f;
 }
 
+// The same in two parts for a kernel that keeps no hit record: an accepted
+// triangle's fields when it is accepted (a later one writes over them, and
+// there are few), Tclosest and a miss's fields at the end of the ray.
+__device__ __forceinline__ void store_found(const HitSoA& hs, uint64_t i, int32_t elem, float U, float V, float W) {
+  if (hs.prim) hs.prim[i] = elem;
+  if (hs.u) hs.u[i] = U;
+  if (hs.v) hs.v[i] = V;
+  if (hs.w) hs.w[i] = W;
+}
+__device__ __forceinline__ void store_end(const HitSoA& hs, uint64_t i, float t, bool hit) {
+  if (hs.geom) hs.geom[i] = -1;
+  if (hs.t) hs.t[i] = t;
+  if (hit) return;
+  store_found(hs, i, -1, 0.0f, 0.0f, 0.0f);
+}
+
 template <bool COUNT>
 __device__ __forceinline__ void flush_counters(DScratch* s, const Counters& c) {
   if (!COUNT) return;
@@ -856,6 +880,21 @@ __global__ void k_jobs_scatter(const JobDesc* jobs, uint32_t n_jobs, uint64_t n,
 // instructions, 19.6 -> 22.9 lanes active, whole call 6.94 -> 6.56 ms; 300,007
 // coherent shadow rays on 200,003 triangles 0.61 -> 0.56 ms; 262,147 rays on
 // 100,000 moving triangles 1.43 -> 1.35 ms.
+
+// Rays a warp holds at once: a launch of fewer rays than lanes spreads them
+// over all its warps (a warp's step takes as long for one lane as for 32, and
+// the cooperative leaf phase then gives a ray all the lanes), and a larger one
+// fills them.  The walk's tail cutoff shrinks with it (8 stragglers
+// among 8 rays would end every walk at its first leaf).
+// 3,072-path room, depth 4: 1.16 -> 0.59 ms a render; 8,192 rays 217 -> 123 us;
+// 65,000 rays 350 -> 307 us; above 32 rays a warp nothing changes.
+__device__ __forceinline__ unsigned warp_quota(uint64_t n, int& walk_tail) {
+  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t per = (n + warps - 1) / warps;
+  const unsigned q = per < 1 ? 1u : (per > 32 ? 32u : (unsigned)per);
+  walk_tail = min(walk_tail, (int)q / 4);
+  return q;
+}
 
 // 32 bytes of read-only global memory (32-byte aligned) as two float4, in
 // one 256-bit load: a node of 128 bytes takes four load instructions
@@ -1226,6 +1265,7 @@ __device__ __forceinline__ int32_t leaf_scan_dispatch(const DMesh& m, TRay& r, u
       default: return leaf_scan<MOTION, 5>(m, r, first, count, tr0, tr1, tm, omt, U, V, W);
     }
   }
+  class_axes(r.cls, r.kx, r.ky, r.kz);
   return leaf_scan<MOTION, -1>(m, r, first, count, tr0, tr1, tm, omt, U, V, W);
 }
 
@@ -1274,11 +1314,7 @@ __device__ __forceinline__ int32_t coop_leaf(const float4* tris, float lower, TR
     q.s0 = __shfl_sync(kFull, r.s0, o);
     q.s1 = __shfl_sync(kFull, r.s1, o);
     q.s2 = __shfl_sync(kFull, r.s2, o);
-    if (C < 0) {
-      q.kx = __shfl_sync(kFull, r.kx, o);
-      q.ky = __shfl_sync(kFull, r.ky, o);
-      q.kz = __shfl_sync(kFull, r.kz, o);
-    }
+    if (C < 0) class_axes(__shfl_sync(kFull, r.cls, o), q.kx, q.ky, q.kz);
     const float4* ot = reinterpret_cast<const float4*>(
         __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(tris), o));
     const float olower = __shfl_sync(kFull, lower, o);
@@ -1345,11 +1381,7 @@ __device__ __forceinline__ int32_t coop_leaf_mix(const float4* t0, const float4*
     q.s0 = __shfl_sync(kFull, r.s0, o);
     q.s1 = __shfl_sync(kFull, r.s1, o);
     q.s2 = __shfl_sync(kFull, r.s2, o);
-    if (C < 0) {
-      q.kx = __shfl_sync(kFull, r.kx, o);
-      q.ky = __shfl_sync(kFull, r.ky, o);
-      q.kz = __shfl_sync(kFull, r.kz, o);
-    }
+    if (C < 0) class_axes(__shfl_sync(kFull, r.cls, o), q.kx, q.ky, q.kz);
     const float4* a0 = reinterpret_cast<const float4*>(
         __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(t0), o));
     const float4* a1 = reinterpret_cast<const float4*>(
@@ -1445,7 +1477,6 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanes_below = (1u << lane) - 1u;
   TRay r;
-  HitRec h{-1, -1, 0.f, 0.f, 0.f};
   // Current entry, popped and not culled; -1 = no entry left.
   int node = -1, sp = 0;
   SlabRay slab{};
@@ -1460,8 +1491,9 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
   uint32_t dkey = 0;  // motion: nodes from the ray's first key to its second (n_nodes, or 0 at a key)
   const float4* tr0 = reinterpret_cast<const float4*>(MOTION ? m.mtris : m.tris);
   const float4* tr1 = tr0;
+  const bool holds = lane < warp_quota(n, walk_tail);  // the lane takes rays
   for (;;) {
-    const unsigned need = __ballot_sync(kFull, !alive);
+    const unsigned need = __ballot_sync(kFull, !alive && holds);
     if (need != 0u && more) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
@@ -1472,7 +1504,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
       }
       base = __shfl_sync(kFull, base, leader);
       if (base + __popc(need) >= n) more = false;
-      if (!alive) {
+      if (!alive && holds) {
         const uint64_t i = base + __popc(need & lanes_below);
         if (i < n) {
           if (!MOTION && rays.rec) {  // the key-ordered copy as records (RaySoA::rec)
@@ -1488,7 +1520,6 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             rid = order ? (uint64_t)__ldg(order + i) : i;
             load_ray(rays, i, r);
           }
-          h = HitRec{-1, -1, 0.f, 0.f, 0.f};
           hit = false;
           node = 0;  // the root, pushed with T = Tclosest (intersect.go:93-95)
           slab = slab_ray(r);
@@ -1506,7 +1537,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             const int key = (int)fk, key2 = (int)ceilf(k);
             if (key < 0 || key2 >= (int)m.keys) {
               // out of the key range: the reference indexes out of bounds; miss
-              store_hit(hits, rid, r, false, h);
+              store_end(hits, rid, r.tclosest, false);
               alive = false;
             } else {
               dkey = key2 != key ? m.n_nodes : 0u;
@@ -1610,10 +1641,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
         float U = 0.f, V = 0.f, W = 0.f;
         const int32_t idx = leaf_scan_dispatch<MOTION>(m, r, first, count, tr0, tr1, tm, omt, U, V, W);
         if (idx != -1) {
-          h.elem = MOTION ? __ldg(m.elem + idx) : idx;
-          h.u = U;
-          h.v = V;
-          h.w = W;
+          store_found(hits, rid, MOTION ? __ldg(m.elem + idx) : idx, U, V, W);
           hit = true;
         }
         if (ANY && idx != -1) {  // shadow rays stop at the first hit leaf (intersect.go:231-236)
@@ -1639,10 +1667,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                                       U, V, W);
       if (has) {
         if (idx != -1) {
-          h.elem = MOTION ? __ldg(m.elem + idx) : idx;
-          h.u = U;
-          h.v = V;
-          h.w = W;
+          store_found(hits, rid, MOTION ? __ldg(m.elem + idx) : idx, U, V, W);
           hit = true;
         }
         if (ANY && idx != -1) {
@@ -1655,7 +1680,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     if (alive) {
       if (!walking && node == -1) done = true;
       if (done) {
-        store_hit(hits, rid, r, hit, h);
+        store_end(hits, rid, r.tclosest, hit);
         alive = false;
         if (status != kStatusOk) {
           atomicMax(&scratch->status, status);
@@ -1727,8 +1752,9 @@ __global__ void __launch_bounds__(128, MOT ? 5 : 7)
   uint64_t li = 0;    // the ray's position in rays (the world ray is reloaded from it)
   float tm_unused = 0.f, omt_unused = 1.f;
   int key_unused = 0, key2_unused = 0;
+  const bool holds = lane < warp_quota(n, walk_tail);  // the lane takes rays
   for (;;) {
-    const unsigned need = __ballot_sync(kFull, !alive);
+    const unsigned need = __ballot_sync(kFull, !alive && holds);
     if (need != 0u && more) {
       const int leader = __ffs(need) - 1;
       unsigned long long b0 = 0;
@@ -1738,7 +1764,7 @@ __global__ void __launch_bounds__(128, MOT ? 5 : 7)
       }
       b0 = __shfl_sync(kFull, b0, leader);
       if (b0 + __popc(need) >= n) more = false;
-      if (!alive) {
+      if (!alive && holds) {
         const uint64_t i = b0 + __popc(need & lanes_below);
         if (i < n) {
           rid = order ? (uint64_t)__ldg(order + i) : i;
