@@ -354,8 +354,9 @@ int launch_trace_chunk(vmr_ctx* ctx, const DMesh* mesh, const vmr_rays& r, size_
     if (!mb) mb = ctx->top.bounds6;
     // A static mesh in the while-while kernel reads the copy as 32-byte
     // records (two 16-byte loads a ray, its input index inside), written
-    // over the order and array regions (4 + 28 bytes a ray).
-    const bool recs = mesh && mesh->keys <= 1 && !r.time && (tn.kernel & vmr::kKernelWhileWhile);
+    // over the order and array regions (4 + 28 bytes a ray); a static mesh reads
+    // no ray times.
+    const bool recs = mesh && mesh->keys <= 1 && (tn.kernel & vmr::kKernelWhileWhile);
     if (recs) sorted = vmr::RaySoA{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, order};
     int se = vmr::launch_ray_sort(l.rays, n, mb, tn.sort_bits ? tn.sort_bits : 4, keys, hist, order, sorted,
                                   ctx->stream);

@@ -157,7 +157,7 @@ extern "C" int vmr_trace_mesh_noalloc(vmr_ctx* ctx, uint32_t geom, const vmr_ray
   if ((tuning.kernel & vmr::kKernelSort) && n >= vmr::kSortMinRays) {
     // a static mesh in the while-while kernel reads the copy as 32-byte
     // records (RaySoA::rec), which fill the ray region exactly
-    const bool recs = mesh->keys <= 1 && !rays->time && (tuning.kernel & vmr::kKernelWhileWhile);
+    const bool recs = mesh->keys <= 1 && (tuning.kernel & vmr::kKernelWhileWhile);
     vmr::RaySoA sorted{f, f + kMaxRays, f + 2 * kMaxRays, f + 3 * kMaxRays, f + 4 * kMaxRays,
                        f + 5 * kMaxRays, f + 6 * kMaxRays, rays->time ? f + 7 * kMaxRays : nullptr};
     if (recs) sorted = vmr::RaySoA{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, f};

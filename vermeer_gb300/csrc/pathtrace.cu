@@ -1342,10 +1342,10 @@ static int render_path_impl(vmr_ctx* ctx, const vmr_path_params* p, float* fb, v
       srt.bounds[k] = glo[k];
       srt.bounds[3 + k] = ghi[k];
     }
-    srt.keys = reinterpret_cast<uint32_t*>(base + o_sort);
+    srt.hist = reinterpret_cast<uint32_t*>(base + o_sort);  // first: the scan reads it in 16-byte words
+    srt.keys = srt.hist + kSortBucketsMax;
     srt.order = srt.keys + cap;
     srt.rays = reinterpret_cast<float*>(srt.order + cap);
-    srt.hist = reinterpret_cast<uint32_t*>(srt.rays + cap * 8);
   }
   // the traversal's view: the scene's top level, or for jobs only the mesh
   // table (each ray enters its own mesh)
