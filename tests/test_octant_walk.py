@@ -119,3 +119,48 @@ def test_ray_counts_around_the_warps_share(ctx, n):
                     assert np.array_equal(x, y), (o, shadow)
     finally:
         ctx.set_tuning()
+
+
+@pytest.mark.parametrize("kind", ["clean", "swapped", "nan", "inf"])
+@pytest.mark.parametrize("moving", [False, True])
+def test_top_level_copies_equal_the_nodes(ctx, kind, moving):
+    """A top level over meshes, a sphere and (moving) motion and transformed
+    meshes, its boxes as an upload may hold them."""
+    from vermeer_gb300 import scenes
+    rng = np.random.default_rng(9)
+    geoms = []
+    for k in range(9):
+        v, ip = scenes.triangle_soup(200 + 90 * k, 50 + k, lo=0.1 * k, hi=0.1 * k + 0.4, edge=0.05)
+        if moving and k % 3 == 1:
+            v = np.concatenate([v, v + np.float32(0.05) * rng.standard_normal(3).astype(np.float32)])
+            geoms.append(ctx.mesh_build(v, ip, keys=2, motion_mode=1))
+        else:
+            geoms.append(ctx.mesh_build(v, ip))
+            if moving and k % 3 == 2:
+                ctx.mesh_set_transform(geoms[-1], [1, 0.1, 0, 0, -0.1, 1, 0, 0, 0, 0, 0.9, 0, 0.05, 0, 0.1, 1])
+    geoms.append(ctx.sphere_add((0.4, 0.5, 0.6), 0.15))
+    ctx.scene_build(geoms)
+    if kind != "clean":
+        e = ctx.scene_export(len(geoms))
+        if e["keys"] == 1:
+            nodes, boxes = e["nodes"].copy(), np.ascontiguousarray(e["nodes"]["boxes"])
+            _spoil(boxes, kind)
+            nodes["boxes"] = boxes
+            ctx.scene_upload(e["geom_order"], nodes=nodes)
+        else:
+            boxes = e["mboxes"].copy()
+            _spoil(boxes, kind)
+            ctx.scene_upload(e["geom_order"], mnodes=e["mnodes"], mboxes=boxes, keys=e["keys"])
+    rays = _rays(4099, 13)
+    try:
+        for shadow in (False, True):
+            got = {}
+            for k in (0, 13, 45):
+                ctx.set_tuning(kernel=k)
+                got[k] = ctx.trace_scene(rays, shadow=shadow)
+            for k in (13, 45):
+                for o in OUT + ("geom",):
+                    x, y = (z[o].view(np.uint32) if z[o].dtype == np.float32 else z[o] for z in (got[k], got[0]))
+                    assert np.array_equal(x, y), (o, k, shadow)
+    finally:
+        ctx.set_tuning()

@@ -138,6 +138,25 @@ cudaError_t octant_nodes(vmr_ctx* ctx, const DevBuf& nodes, uint32_t n, DevBuf& 
   return e;
 }
 
+// The octant copies of a motion tree; *bad_dev: the device flag that says whether
+// they may be used (null: there are none, and the traces walk the mnodes).
+cudaError_t octant_mnodes(vmr_ctx* ctx, const DevBuf& mnodes, const DevBuf& mboxes, uint32_t keys, uint32_t n,
+                          DevBuf& buf, int*& bad_dev) {
+  bad_dev = nullptr;
+  // an index plus the keys' offset stays below the kernels' markers
+  if (n == 0 || (uint64_t)8 * keys * n >= 0xfffffffeull) return cudaSuccess;
+  const size_t bytes = (size_t)8 * keys * n * sizeof(vmr::ONode);
+  cudaError_t e = buf.ensure(bytes + 16);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  if (e != cudaSuccess) return e;
+  bad_dev = reinterpret_cast<int*>(buf.as<char>() + bytes);
+  return (cudaError_t)vmr::launch_octant_mnodes(mnodes.as<MNode>(), mboxes.p, keys, n, buf.as<vmr::ONode>(), bad_dev,
+                                                ctx->stream);
+}
+
 // Host accelerator -> device arrays (layout in device.h).  tris_ready: the
 // device builder already wrote the static triangle table into rec.tris.
 int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
@@ -188,22 +207,7 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
     VMR_CUDA(ctx, upload(ctx, rec.mtris, tris));
     VMR_CUDA(ctx, upload(ctx, rec.elem, elem));
     const uint32_t nm = (uint32_t)m.mnodes.size();
-    // obase + keys * n_nodes stays in 32 bits (the kernels' index)
-    if ((uint64_t)8 * m.keys * nm < 0xfffffffeull) {
-      const size_t ob = (size_t)8 * m.keys * nm * sizeof(vmr::ONode);
-      const cudaError_t e = rec.onodes.ensure(ob + 16);
-      if (e == cudaSuccess) {
-        int* flag = reinterpret_cast<int*>(rec.onodes.as<char>() + ob);
-        const int le = vmr::launch_octant_mnodes(rec.mnodes.as<MNode>(), rec.mboxes.p, m.keys, nm,
-                                                 rec.onodes.as<vmr::ONode>(), flag, ctx->stream);
-        if (le != 0) return cuda_fail(ctx, (cudaError_t)le, "octant nodes launch");
-        bad_dev = flag;
-      } else if (e == cudaErrorMemoryAllocation) {  // the traces walk mnodes
-        cudaGetLastError();
-      } else {
-        return cuda_fail(ctx, e, "octant nodes");
-      }
-    }
+    VMR_CUDA(ctx, octant_mnodes(ctx, rec.mnodes, rec.mboxes, m.keys, nm, rec.onodes, bad_dev));
     d.n_nodes = nm;
     d.mnodes = rec.mnodes.as<MNode>();
     d.mboxes = rec.mboxes.p;
@@ -248,12 +252,15 @@ int refresh_top(vmr_ctx* ctx) {
   for (size_t i = 0; i < ctx->meshes.size(); ++i) table[i] = ctx->meshes[i]->dmesh;
   VMR_CUDA(ctx, upload(ctx, t.meshes, table));
   DTop d{};
+  int* bad_dev = nullptr;
   if (t.host.keys <= 1) {
     std::vector<GNode> g;
     if (!repack_nodes(t.host.nodes, (uint32_t)t.host.geom_order.size(), g))
       return fail(ctx, VMR_ERR_INVALID, "malformed top-level nodes");
     VMR_CUDA(ctx, upload(ctx, t.nodes, g));
     d.nodes = t.nodes.as<GNode>();
+    d.n_nodes = (uint32_t)t.host.nodes.size();
+    VMR_CUDA(ctx, octant_nodes(ctx, t.nodes, d.n_nodes, t.onodes, d.onodes));
     d.keys = 1;
     d.iter_cap = 4u * (uint32_t)t.host.nodes.size() + 2u;
   } else {
@@ -267,9 +274,14 @@ int refresh_top(vmr_ctx* ctx) {
     d.keys = t.host.keys;
     d.n_mnodes = (uint32_t)t.host.mnodes.size();
     d.iter_cap = 4u * (uint32_t)t.host.mnodes.size() + 2u;
+    d.n_nodes = d.n_mnodes;
+    VMR_CUDA(ctx, octant_mnodes(ctx, t.mnodes, t.mboxes, d.keys, d.n_mnodes, t.onodes, bad_dev));
   }
   VMR_CUDA(ctx, upload(ctx, t.order, t.host.geom_order));
+  int bad = 0;
+  if (bad_dev) VMR_CUDA(ctx, cudaMemcpyAsync(&bad, bad_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (bad_dev && !bad) d.onodes = t.onodes.as<vmr::ONode>();
   d.geom_order = t.order.as<uint32_t>();
   d.meshes = t.meshes.as<DMesh>();
   d.n_geoms = (uint32_t)t.host.geom_order.size();

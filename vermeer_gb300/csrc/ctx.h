@@ -128,7 +128,7 @@ struct GuideState {
 
 struct TopRec {
   HostTop host;
-  DevBuf nodes, mnodes, mboxes, order, meshes;
+  DevBuf nodes, onodes, mnodes, mboxes, order, meshes;
   DTop dtop{};
   float bounds6[6] = {0, 0, 0, 0, 0, 0};  // union of the geoms' bounds (ray reordering)
   bool valid = false;

@@ -107,6 +107,9 @@ enum MeshKind : uint32_t { kTriangles = 0, kSphere = 1, kGroup = 2 };
 // boxes; leaves index geom_order (leaf position -> geom id).
 struct DTop {
   const GNode* nodes;
+  const ONode* onodes;      // as DMesh::onodes, of the top level
+  uint32_t n_nodes;
+  uint32_t pad0;
   const MNode* mnodes;
   const void* mboxes;
   const uint32_t* geom_order;

@@ -1419,6 +1419,8 @@ static int render_path_impl(vmr_ctx* ctx, const vmr_path_params* p, float* fb, v
     fold(b.env, sizeof(b.env));
     fold(&b.sel, sizeof(b.sel));
     fold(&top, sizeof(top));
+    if (flat.mesh) fold(flat.mesh, sizeof(*flat.mesh));  // a later scene's flat mesh may come to the same address
+    fold(&flat.n, sizeof(flat.n));
     const uint64_t nj = b.n_jobs;
     fold(&nj, sizeof(nj));
     fold(&b.alpha, sizeof(b.alpha));

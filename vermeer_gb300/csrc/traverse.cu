@@ -1158,6 +1158,15 @@ __device__ __forceinline__ bool push_slots(S& stk, int& sp, const Slots& o, int&
   return true;
 }
 
+struct ArrayStack {
+  int2* e;
+  __device__ __forceinline__ void set(int i, int node, float T) { e[i] = make_int2(node, __float_as_int(T)); }
+};
+__device__ __forceinline__ bool push_slots_at(int2* stk, int& sp, const Slots& o, int& next, int& status) {
+  ArrayStack a{stk};
+  return push_slots(a, sp, o, next, status);
+}
+
 // The visit of the node itself (b: its boxes, at the ray's time for a motion
 // node): meshes without octant copies, and (exact) rays whose slab test can
 // meet a NaN, with the reference's MINPS/MAXPS operand order.  The children to
@@ -1716,12 +1725,20 @@ __device__ __forceinline__ bool motion_keys(uint32_t keys, float time, float& tm
   return !(key < 0 || key2 >= (int)keys);
 }
 
-// Capped for 7 resident blocks per SM (72 registers; the two-level sphere
-// grid 1% faster than at 8).  MOT (motion meshes and top levels) holds more
-// state: capped for 5 (96 registers) instead, as at 8 it spilled 1 KB per
-// thread and measured 27% slower on the batched jobs.
+// The walk is k_trace_mesh_ww's: octant copies of the current level's nodes,
+// pops in the visit's step.  What a lane needs between levels only (the
+// mesh's triangles and lower bound, the ray's own direction) is read again
+// where it is needed instead of held.
+//
+// Bound as that kernel is.  Register caps, measured (1,000,003 rays on the
+// sphere grid; 16 path jobs, half of them moving): static scenes 6 blocks per SM
+// 495 us, 7 503, 8 517; MOT 4 blocks 6.55 ms, 5 6.64, 6 6.94.  Against the walk
+// over the nodes: scene 517 -> 495 us, room render 5.90 -> 5.73 ms, path jobs
+// 6.65 -> 6.55 ms.
+enum SceneLevel : int { kLevelStatic = 0, kLevelMotion = 1, kLevelNodes = 2 };
+
 template <bool ANY, bool COOP = false, bool MOT = false>
-__global__ void __launch_bounds__(128, MOT ? 5 : 7)
+__global__ void __launch_bounds__(128, MOT ? 4 : 6)
     k_trace_scene_ww(const DTop top, RaySoA rays, HitSoA hits, uint64_t n, DScratch* scratch,
                      const unsigned long long* n_dev, const uint32_t* order, int walk_tail,
                      const uint32_t* ray_path, const uint32_t* path_geom) {
@@ -1733,80 +1750,157 @@ __global__ void __launch_bounds__(128, MOT ? 5 : 7)
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanes_below = (1u << lane) - 1u;
   TRay r;
-  HitRec h{-1, -1, 0.f, 0.f, 0.f};
+  SlabRay slab{};
   int node = -1, sp = 0;
-  float nodeT = 0.f;
-  uint64_t rid = 0;
-  uint32_t iter = 0, miter = 0;
+  uint64_t li = 0;  // the ray's position in rays
+  uint32_t iter = 0, miter = 0;  // visits left in the top level, in the mesh
   bool alive = false, hit = false, more = true;
+  bool need = false;  // the lane's next entry is to be found (next_entry)
   int status = kStatusOk;
   // current mesh (geom >= 0) and the top-level leaf's remaining geoms
   int geom = -1, base = 0;
   uint32_t leaf_next = 0, leaf_left = 0;
-  const GNode* mnodes = nullptr;
-  const float4* mtris = nullptr;
-  float lower = 0.f;
-  uint32_t mcap = 0;
-  bool mmot = false;  // the current mesh has motion keys (its key data is re-read from top.meshes)
-  bool mxf = false;   // the current mesh has a transform: r is its object-space ray
-  uint64_t li = 0;    // the ray's position in rays (the world ray is reloaded from it)
-  float tm_unused = 0.f, omt_unused = 1.f;
-  int key_unused = 0, key2_unused = 0;
+  // the current level's nodes for this ray: the octant copy (level static or
+  // motion: from its first key, dkey nodes on to its second, weight tm)
+  const ONode* on = nullptr;
+  int level = kLevelNodes;
+  uint32_t dkey = 0;
+  float tm = 0.f;
+  bool mxf = false;  // the current mesh has a transform: r is its object-space ray
+
+  // The level of a static (keys 1) or motion tree; false outside its keys.
+  auto enter = [&](const ONode* onodes, uint32_t n_nodes, uint32_t keys) -> bool {
+    on = onodes;
+    level = r.exact || !onodes ? kLevelNodes : kLevelStatic;
+    uint32_t o = r.oct;
+    if (MOT && keys > 1) {
+      float omt;
+      int key, key2;
+      if (!motion_keys(keys, r.time, tm, omt, key, key2)) return false;
+      dkey = key2 != key ? n_nodes : 0u;
+      o = o * keys + (uint32_t)key;
+      if (level == kLevelStatic) level = kLevelMotion;
+    }
+    on += (size_t)o * n_nodes;
+    return true;
+  };
+  auto world_ray = [&]() {  // the ray of the stream, its Tclosest and time kept
+    load_ray_pd(rays, li, r);
+    slab = slab_ray(r);
+  };
+  auto sphere = [&](const DMesh& M, uint32_t g) {  // an analytic sphere: tested here, no stack
+    TRay w;
+    w.ox = __ldg(rays.px + li); w.oy = __ldg(rays.py + li); w.oz = __ldg(rays.pz + li);
+    w.dx = __ldg(rays.dx + li); w.dy = __ldg(rays.dy + li); w.dz = __ldg(rays.dz + li);
+    w.tclosest = r.tclosest;
+    HitRec h;
+    if (!sphere_hit(M, w, h)) return;
+    r.tclosest = w.tclosest;
+    hit = true;
+    const uint64_t rid = order ? (uint64_t)__ldg(order + li) : li;
+    store_found(hits, rid, 0, 0.0f, 0.0f, 0.0f);
+    if (hits.geom) hits.geom[rid] = (int)g;
+  };
+  // Mesh g at its root, pushed with T = Tclosest; false: nothing to walk.
+  auto enter_mesh = [&](uint32_t g) -> bool {
+    const DMesh& M = top.meshes[g];
+    if (M.kind == kSphere) {
+      sphere(M, g);
+      return false;
+    }
+    if (M.n_tris == 0) return false;
+    mxf = MOT && M.has_xf;
+    if (mxf) {
+      world_ray();
+      ray_to_object(r, M.xf_inv);
+      slab = slab_ray(r);
+    }
+    if (!enter(M.onodes, M.n_nodes, M.keys)) {
+      if (mxf) world_ray();
+      mxf = false;
+      return false;
+    }
+    geom = (int)g;
+    miter = M.iter_cap;
+    node = 0;
+    return true;
+  };
+  // The next entry the reference does not cull when it pops it: the mesh's
+  // own, the next geom of the top-level leaf, the top level's; -1: none.
+  auto next_entry = [&]() {
+    for (;;) {
+      if (geom >= 0) {
+        while (sp > base) {
+          const int2 e = stk[--sp];
+          if (!(r.tclosest < __int_as_float(e.y))) {  // intersect.go:106
+            node = e.x;
+            return;
+          }
+        }
+        geom = -1;  // the mesh traversal is done
+        sp = base - 1;
+        if (MOT && mxf) {
+          world_ray();
+          mxf = false;
+        }
+        if (!ray_path) enter(top.onodes, top.n_nodes, top.keys);
+      }
+      node = -1;
+      if (leaf_left > 0) {
+        const uint32_t g = __ldg(top.geom_order + leaf_next);
+        ++leaf_next;
+        --leaf_left;
+        if (enter_mesh(g)) {
+          base = sp + 1;
+          sp = base;
+          if (base >= kStackCapacity) status = kStatusStackOverflow;
+          return;
+        }
+        if (ANY && hit) return;
+        continue;
+      }
+      if (ANY && hit) return;  // shadow rays stop after the leaf that hit (intersect.go:231-236)
+      if (sp == 0) return;
+      const int2 e = stk[--sp];
+      if (r.tclosest < __int_as_float(e.y)) continue;
+      node = e.x;
+      if (node >= 0) return;
+      leaf_decode(node, leaf_next, leaf_left);  // a top-level leaf: its geoms, in order
+    }
+  };
+
   const bool holds = lane < warp_quota(n, walk_tail);  // the lane takes rays
   for (;;) {
-    const unsigned need = __ballot_sync(kFull, !alive && holds);
-    if (need != 0u && more) {
-      const int leader = __ffs(need) - 1;
+    const unsigned idle = __ballot_sync(kFull, !alive && holds);
+    if (idle != 0u && more) {
+      const int leader = __ffs(idle) - 1;
       unsigned long long b0 = 0;
       if ((int)lane == leader) {
-        b0 = atomicAdd(&scratch->next_ray, (unsigned long long)__popc(need));
+        b0 = atomicAdd(&scratch->next_ray, (unsigned long long)__popc(idle));
         if (*reinterpret_cast<volatile int*>(&scratch->status) != kStatusOk) b0 = n;
       }
       b0 = __shfl_sync(kFull, b0, leader);
-      if (b0 + __popc(need) >= n) more = false;
+      if (b0 + __popc(idle) >= n) more = false;
       if (!alive && holds) {
-        const uint64_t i = b0 + __popc(need & lanes_below);
+        const uint64_t i = b0 + __popc(idle & lanes_below);
         if (i < n) {
-          rid = order ? (uint64_t)__ldg(order + i) : i;
           li = i;
           load_ray(rays, i, r);
-          h = HitRec{-1, -1, 0.f, 0.f, 0.f};
+          slab = slab_ray(r);
           hit = false;
-          node = 0;  // the top-level root, pushed with T = Tclosest
-          nodeT = r.tclosest;
+          node = -1;
           sp = 0;
-          iter = 0;
+          iter = top.iter_cap;
           geom = -1;
           leaf_left = 0;
           alive = true;
+          need = false;
           if (ray_path) {  // job mode: enter the ray's own mesh, as a top-level leaf would
-            const uint32_t g = __ldg(path_geom + __ldg(ray_path + rid));
-            const DMesh& M = top.meshes[g];
-            if (M.kind == 1) {  // an analytic sphere: tested here
-              if (sphere_hit(M, r, h)) {
-                h.geom = (int)g;
-                hit = true;
-              }
-              node = -1;
-            } else if (M.n_tris == 0) {
-              node = -1;
-            } else if (MOT && M.keys > 1 && !motion_keys(M.keys, r.time, tm_unused, omt_unused, key_unused, key2_unused)) {
-              node = -1;
-            } else {
-              base = 1;
-              geom = (int)g;
-              mmot = MOT && M.keys > 1;
-              if (MOT && M.has_xf) ray_to_object(r, M.xf_inv);  // the mesh is the ray's whole walk
-              mnodes = M.nodes;
-              mtris = reinterpret_cast<const float4*>(M.tris);
-              lower = M.lower_static;
-              mcap = M.iter_cap;
-              miter = 0;
-              sp = base;
-            }
-          } else if (MOT && top.keys > 1 && !motion_keys(top.keys, r.time, tm_unused, omt_unused, key_unused,
-                                                         key2_unused)) {
-            node = -1;  // outside the top level's key range: a miss
+            const uint64_t rid = order ? (uint64_t)__ldg(order + i) : i;
+            base = 1;
+            if (enter_mesh(__ldg(path_geom + __ldg(ray_path + rid)))) sp = base;
+          } else if (enter(top.onodes, top.n_nodes, top.keys)) {  // outside the top level's keys: a miss
+            node = 0;  // the top-level root, pushed with T = Tclosest
           }
         }
       }
@@ -1818,7 +1912,7 @@ __global__ void __launch_bounds__(128, MOT ? 5 : 7)
     }
     bool done = false, walking = false;
     if (alive) {
-      walking = node != -1;
+      walking = need || node >= 0;
       for (;;) {
         const unsigned wmask = __ballot_sync(alive_mask, walking);
         if (wmask == 0u) break;
@@ -1826,280 +1920,128 @@ __global__ void __launch_bounds__(128, MOT ? 5 : 7)
           // a leaf for the cooperative scan ends the walk early; without it
           // (COOP off) a motion leaf is scanned by its own lane, and a walk
           // cut short for it idles the warp
-          const unsigned leafy = __ballot_sync(alive_mask, !walking && node < -1 && geom >= 0 && !(MOT && mmot && !COOP));
+          const unsigned leafy = __ballot_sync(alive_mask, !walking && node < -1 && !(MOT && !COOP && level != kLevelStatic));
           if (leafy != 0u) break;
         }
         if (!walking) continue;
-        if (geom < 0 ? ++iter > top.iter_cap : ++miter > mcap) {
-          status = kStatusIterationCap;
-          done = true;
-          walking = false;
-          continue;
-        }
-        // next entry: a pop, the next geom of the leaf, or the end
-        bool need_pop = false;
-        if (r.tclosest < nodeT) {  // pop-time cull (intersect.go:106)
-          need_pop = true;
-        } else if (node >= 0) {
-          float4 b[6];
-          int4 ch;
-          unsigned rk;
-          if (MOT && geom >= 0 && mmot) {  // a motion mesh: boxes lerped at the ray's time
-            const DMesh& M = top.meshes[geom];
-            float tm, omt;
-            int key, key2;
-            motion_keys(M.keys, r.time, tm, omt, key, key2);
-            const float4* bx = reinterpret_cast<const float4*>(M.mboxes);
-            fetch_mnode(M.mnodes, node, r.oct, bx + (size_t)key * M.n_mnodes * 6, bx + (size_t)key2 * M.n_mnodes * 6, tm,
-                        omt, b, ch, rk);
-          } else if (MOT && geom < 0 && top.keys > 1) {  // a motion top level
-            float tm, omt;
-            int key, key2;
-            motion_keys(top.keys, r.time, tm, omt, key, key2);
-            const float4* bx = reinterpret_cast<const float4*>(top.mboxes);
-            fetch_mnode(top.mnodes, node, r.oct, bx + (size_t)key * top.n_mnodes * 6,
-                        bx + (size_t)key2 * top.n_mnodes * 6, tm, omt, b, ch, rk);
+        if (!need) {
+          if (geom < 0 ? iter-- == 0u : miter-- == 0u) {
+            status = kStatusIterationCap;
           } else {
-            const GNode* nb = geom < 0 ? top.nodes : mnodes;
-            uint4 meta;
-            ld_node(nb + node, b, ch, meta);
-            rk = (((r.oct & 4u) ? meta.z : meta.y) >> ((r.oct & 3u) * 8u)) & 0xffu;
-          }
-          float tn[4];
-          unsigned mask = r.exact ? box4<true>(r, b, tn) : box4<false>(r, b, tn);
-          if (ch.x == kEmptyChild || r.tclosest < tn[0]) mask &= ~1u;
-          if (ch.y == kEmptyChild || r.tclosest < tn[1]) mask &= ~2u;
-          if (ch.z == kEmptyChild || r.tclosest < tn[2]) mask &= ~4u;
-          if (ch.w == kEmptyChild || r.tclosest < tn[3]) mask &= ~8u;
-          int next = 0;
-          float nextT = 0.f;
-          if (push_ranked(stk, sp, mask, ch, tn, rk, next, nextT, status)) {
-            node = next;
-            nodeT = nextT;
-            continue;
-          }
-          if (status != kStatusOk) {
-            done = true;
-            walking = false;
-            continue;
-          }
-          need_pop = true;
-        } else if (node == kEmptyChild) {
-          need_pop = true;
-        } else if (geom >= 0) {  // a mesh leaf: the leaf phase scans it
-          walking = false;
-          continue;
-        } else {  // a top-level leaf: its geoms, in order
-          uint32_t first, count;
-          leaf_decode(node, first, count);
-          leaf_next = first;
-          leaf_left = count;
-          need_pop = true;  // handled below: enter the first geom
-        }
-        // pop / enter the next geom / leave a finished mesh
-        for (;;) {
-          if (geom >= 0 && sp > base) {  // the mesh's own entries
-            const int2 e = stk[--sp];
-            node = e.x;
-            nodeT = __int_as_float(e.y);
-            break;
-          }
-          if (geom >= 0) {  // the mesh traversal is done
-            geom = -1;
-            sp = base - 1;
-            if (MOT && mxf) {  // back to the world ray (Tclosest kept)
-              load_ray_pd(rays, li, r);
-              mxf = false;
-            }
-          }
-          if (leaf_left > 0) {  // enter the next geom of the top-level leaf
-            const uint32_t g = __ldg(top.geom_order + leaf_next);
-            ++leaf_next;
-            --leaf_left;
-            const DMesh& M = top.meshes[g];
-            if (M.kind == 1) {  // an analytic sphere: tested here, no stack
-              if (sphere_hit(M, r, h)) {
-                h.geom = (int)g;
-                hit = true;
-                if (ANY) {
-                  node = -1;
-                  break;
-                }
+            int next = 0;
+            bool pushed = false;
+            if (level != kLevelNodes) {
+              Slots o;
+              if (MOT && level == kLevelMotion) {
+                const float omt = __fsub_rn(1.0f, tm);
+                visit_octant_m(on + node, on + node + dkey, slab, pack2(tm, tm), pack2(omt, omt), r.tclosest, o);
+              } else {
+                visit_octant(on + node, slab, r.tclosest, o);
               }
-              continue;
+              pushed = push_slots_at(stk, sp, o, next, status);
+            } else {
+              float4 b[6];
+              int4 ch;
+              unsigned rk;
+              const uint32_t keys = geom >= 0 ? top.meshes[geom].keys : top.keys;
+              if (MOT && keys > 1) {
+                float t, omt;
+                int key, key2;
+                motion_keys(keys, r.time, t, omt, key, key2);
+                const uint32_t nm = geom >= 0 ? top.meshes[geom].n_mnodes : top.n_mnodes;
+                const float4* bx = reinterpret_cast<const float4*>(geom >= 0 ? top.meshes[geom].mboxes : top.mboxes);
+                fetch_mnode(geom >= 0 ? top.meshes[geom].mnodes : top.mnodes, node, r.oct, bx + (size_t)key * nm * 6,
+                            bx + (size_t)key2 * nm * 6, t, omt, b, ch, rk);
+              } else {
+                uint4 meta;
+                ld_node((geom >= 0 ? top.meshes[geom].nodes : top.nodes) + node, b, ch, meta);
+                rk = (((r.oct & 4u) ? meta.z : meta.y) >> ((r.oct & 3u) * 8u)) & 0xffu;
+              }
+              int2 e[4];
+              const int np = visit_node(b, ch, rk, slab, r.exact, r.tclosest, e);
+              if (sp + np - 1 > kStackCapacity) {
+                status = kStatusStackOverflow;
+              } else if (np > 0) {
+                for (int k = 0; k + 1 < np; ++k) stk[sp++] = e[k];
+                next = e[np - 1].x;
+                pushed = true;
+              }
             }
-            if (M.n_tris == 0) continue;
-            if (MOT && M.keys > 1 && !motion_keys(M.keys, r.time, tm_unused, omt_unused, key_unused, key2_unused)) continue;
-            base = sp + 1;
-            if (base >= kStackCapacity) {
-              status = kStatusStackOverflow;
-              break;
+            node = next;
+            need = !pushed;
+            if (pushed && node < 0 && geom < 0) {  // a top-level leaf
+              leaf_decode(node, leaf_next, leaf_left);
+              need = true;
             }
-            geom = (int)g;
-            mmot = MOT && M.keys > 1;
-            mxf = MOT && M.has_xf;
-            if (mxf) ray_to_object(r, M.xf_inv);
-            mnodes = M.nodes;
-            mtris = reinterpret_cast<const float4*>(M.tris);
-            lower = M.lower_static;
-            mcap = M.iter_cap;
-            miter = 0;
-            sp = base;
-            node = 0;
-            nodeT = r.tclosest;
-            break;
           }
-          if (hit && ANY) {  // shadow rays stop after the leaf that hit (intersect.go:231-236)
-            node = -1;
-            break;
-          }
-          if (sp == 0) {
-            node = -1;
-            break;
-          }
-          const int2 e = stk[--sp];
-          node = e.x;
-          nodeT = __int_as_float(e.y);
-          break;
         }
-        if (status != kStatusOk) {
-          done = true;
-          walking = false;
-          continue;
-        }
-        (void)need_pop;
-        if (node == -1) walking = false;
+        if (need && status == kStatusOk) next_entry();
+        need = false;
+        done = status != kStatusOk;
+        walking = !done && node >= 0;
       }
     }
     // ---- leaf phase: a mesh leaf, scanned in the reference's order (COOP:
     // the warp's leaves as one list of triangle tests, all lanes)
-    const bool any_leaf = alive && !done && !walking && node < -1 && geom >= 0;
-    int32_t cidx = -1;
-    float cU = 0.f, cV = 0.f, cW = 0.f;
-    if (COOP && MOT) {  // static and motion leaves in one cooperative list
+    const bool any_leaf = alive && !done && !walking && node < -1;
+    int32_t idx = -1;
+    float U = 0.f, V = 0.f, W = 0.f;
+    {
       uint32_t first = 0, count = 0;
-      const float4* t0 = mtris;
-      const float4* t1 = mtris;
-      float tm = 0.f, omt = 1.f, lo = lower;
+      const float4* t0 = nullptr;
+      const float4* t1 = nullptr;
+      float lm = 0.f, lomt = 1.f, lo = 0.f;
+      bool mot = false;
+      const DMesh* M = nullptr;
       if (any_leaf) {
         leaf_decode(node, first, count);
-        if (mmot) {
-          const DMesh& M = top.meshes[geom];
+        M = top.meshes + geom;
+        mot = MOT && M->keys > 1;
+        if (mot) {
           int key, key2;
-          motion_keys(M.keys, r.time, tm, omt, key, key2);
-          const float4* tr = reinterpret_cast<const float4*>(M.mtris);
-          t0 = tr + (size_t)key * M.n_tris * 3;
-          t1 = tr + (size_t)key2 * M.n_tris * 3;
-          lo = M.ray_bias;
+          motion_keys(M->keys, r.time, lm, lomt, key, key2);
+          const float4* tr = reinterpret_cast<const float4*>(M->mtris);
+          t0 = tr + (size_t)key * M->n_tris * 3;
+          t1 = tr + (size_t)key2 * M->n_tris * 3;
+          lo = M->ray_bias;
+        } else {
+          t0 = t1 = reinterpret_cast<const float4*>(M->tris);
+          lo = M->lower_static;
         }
       }
-      cidx = coop_leaf_mix_dispatch(t0, t1, tm, omt, any_leaf && mmot, lo, r, any_leaf, first, count, cU, cV, cW);
-    } else if (COOP) {
-      uint32_t first = 0, count = 0;
-      if (any_leaf) leaf_decode(node, first, count);
-      cidx = coop_leaf_dispatch(mtris, lower, r, any_leaf, first, count, cU, cV, cW);
+      if (COOP && MOT) {  // static and motion leaves in one cooperative list
+        idx = coop_leaf_mix_dispatch(t0, t1, lm, lomt, mot, lo, r, any_leaf, first, count, U, V, W);
+      } else if (COOP) {
+        idx = coop_leaf_dispatch(t0, lo, r, any_leaf, first, count, U, V, W);
+      } else if (any_leaf) {
+        if (mot) {  // vertices lerped at the ray's time, scanned by its lane
+          idx = leaf_scan_dispatch<true>(*M, r, first, count, t0, t1, lm, lomt, U, V, W);
+        } else {
+          idx = leaf_scan_dispatch<false>(*M, r, first, count, t0, t0, 0.f, 1.f, U, V, W);
+        }
+      }
+      if (any_leaf) {
+        need = true;  // the rest of the mesh, then the leaf's next geom or the top level
+        if (idx != -1) {
+          const uint64_t rid = order ? (uint64_t)__ldg(order + li) : li;
+          store_found(hits, rid, mot ? __ldg(M->elem + idx) : idx, U, V, W);
+          if (hits.geom) hits.geom[rid] = geom;
+          hit = true;
+          if (ANY) done = true;
+        }
+      }
     }
     if (alive) {
-      if (any_leaf) {
-        uint32_t first, count;
-        leaf_decode(node, first, count);
-        float U = cU, V = cV, W = cW;
-        int32_t idx = cidx;
-        int32_t elem = idx;
-        if (COOP && MOT && mmot) {  // scanned cooperatively: the leaf position to ElemID
-          elem = idx != -1 ? __ldg(top.meshes[geom].elem + idx) : -1;
-        } else if (MOT && mmot) {  // a motion leaf: vertices lerped at the ray's time, scanned by its lane
-          const DMesh& M = top.meshes[geom];
-          float tm, omt;
-          int key, key2;
-          motion_keys(M.keys, r.time, tm, omt, key, key2);
-          const float4* tr = reinterpret_cast<const float4*>(M.mtris);
-          idx = leaf_scan_dispatch<true>(M, r, first, count, tr + (size_t)key * M.n_tris * 3,
-                                         tr + (size_t)key2 * M.n_tris * 3, tm, omt, U, V, W);
-          elem = idx != -1 ? __ldg(M.elem + idx) : -1;
-        } else if (!COOP) {
-          DMesh M;
-          M.lower_static = lower;
-          idx = leaf_scan_dispatch<false>(M, r, first, count, mtris, mtris, 0.f, 1.f, U, V, W);
-          elem = idx;
-        }
-        if (idx != -1) {
-          h.elem = elem;
-          h.geom = geom;
-          h.u = U;
-          h.v = V;
-          h.w = W;
-          hit = true;
-        }
-        if (ANY && idx != -1) {
-          done = true;
-        } else {
-          // the rest of the mesh, then the leaf's next geom or the top level
-          for (;;) {
-            if (sp > base) {
-              const int2 e = stk[--sp];
-              node = e.x;
-              nodeT = __int_as_float(e.y);
-              break;
-            }
-            geom = -1;
-            sp = base - 1;
-            if (MOT && mxf) {  // back to the world ray (Tclosest kept)
-              load_ray_pd(rays, li, r);
-              mxf = false;
-            }
-            if (leaf_left > 0) {
-              const uint32_t g = __ldg(top.geom_order + leaf_next);
-              ++leaf_next;
-              --leaf_left;
-              const DMesh& MM = top.meshes[g];
-              if (MM.kind == 1) {
-                if (sphere_hit(MM, r, h)) {
-                  h.geom = (int)g;
-                  hit = true;
-                  if (ANY) {
-                    node = -1;
-                    break;
-                  }
-                }
-                continue;
-              }
-              if (MM.n_tris == 0) continue;
-              if (MOT && MM.keys > 1 && !motion_keys(MM.keys, r.time, tm_unused, omt_unused, key_unused, key2_unused)) continue;
-              base = sp + 1;
-              geom = (int)g;
-              mmot = MOT && MM.keys > 1;
-              mxf = MOT && MM.has_xf;
-              if (mxf) ray_to_object(r, MM.xf_inv);
-              mnodes = MM.nodes;
-              mtris = reinterpret_cast<const float4*>(MM.tris);
-              lower = MM.lower_static;
-              mcap = MM.iter_cap;
-              miter = 0;
-              sp = base;
-              node = 0;
-              nodeT = r.tclosest;
-              break;
-            }
-            if (hit && ANY) {
-              node = -1;
-              break;
-            }
-            if (sp == 0) {
-              node = -1;
-              break;
-            }
-            const int2 e = stk[--sp];
-            node = e.x;
-            nodeT = __int_as_float(e.y);
-            break;
-          }
-        }
-      }
-      if (!walking && node == -1) done = true;
+      if (!walking && !need && node == -1) done = true;
       if (done) {
-        store_hit(hits, rid, r, hit, h);
+        const uint64_t rid = order ? (uint64_t)__ldg(order + li) : li;
+        if (hits.t) hits.t[rid] = r.tclosest;
+        if (!hit) {
+          store_found(hits, rid, -1, 0.0f, 0.0f, 0.0f);
+          if (hits.geom) hits.geom[rid] = -1;
+        }
         alive = false;
+        need = false;
         if (status != kStatusOk) {
           atomicMax(&scratch->status, status);
           status = kStatusOk;
