@@ -164,3 +164,48 @@ def test_top_level_copies_equal_the_nodes(ctx, kind, moving):
                     assert np.array_equal(x, y), (o, k, shadow)
     finally:
         ctx.set_tuning()
+
+
+@pytest.mark.parametrize("keys", [1, 2, 3])
+@pytest.mark.parametrize("tris", [40, 3000])
+def test_rays_at_box_corners_equal_the_nodes(ctx, keys, tris):
+    """Rays aimed at the vertices of axis-aligned right triangles, whose
+    vertices are their boxes' corners: whether such a ray meets the box, and
+    which triangle it hits, is decided by the last bit of every slab and edge
+    product (and, with motion, of every lerp)."""
+    from vermeer_gb300 import scenes
+    rng = np.random.default_rng(17)
+    c = rng.random((tris, 1, 3))
+    off = rng.choice([-1.0, 1.0], (tris, 3)) * rng.uniform(0.02, 0.12, (tris, 3))
+    ax = rng.integers(0, 3, tris)
+    v = np.repeat(c, 3, 1)
+    k = np.arange(tris)
+    v[k, 1, ax] += off[k, ax]
+    v[k, 2, (ax + 1) % 3] += off[k, (ax + 1) % 3]
+    v = [(v + 0.3 * q * rng.standard_normal((tris, 1, 3))).astype(np.float32) for q in range(keys)]
+    g = ctx.mesh_build(np.concatenate([x.reshape(-1, 3) for x in v]), np.arange(3 * tris, dtype=np.uint32), keys=keys,
+                       motion_mode=1)
+    n = 200_000
+    time = rng.random(n).astype(np.float32)
+    t = time * np.float32(keys - 1)
+    k0 = np.floor(t).astype(int)
+    f = (t - k0).astype(np.float32)[:, None]
+    tri, vert = rng.integers(0, tris, n), rng.integers(0, 3, n)
+    V = np.stack(v)
+    p = (np.float32(1) - f) * V[k0, tri, vert] + f * V[np.minimum(k0 + 1, keys - 1), tri, vert]
+    o = (p + rng.standard_normal((n, 3)).astype(np.float32)).astype(np.float32)
+    rays = np.empty((n, 8), np.float32)
+    rays[:, 0:3], rays[:, 3:6], rays[:, 6], rays[:, 7] = o, p - o, np.inf, time
+    try:
+        for shadow in (False, True):
+            got = {}
+            for k in (0, 13, 45):
+                ctx.set_tuning(kernel=k)
+                got[k] = ctx.trace_mesh(g, rays, shadow=shadow)
+            for k in (13, 45):
+                for q in OUT:
+                    x, y = (z[q].view(np.uint32) if z[q].dtype == np.float32 else z[q] for z in (got[k], got[0]))
+                    bad = np.nonzero(x != y)[0]
+                    assert bad.size == 0, (q, k, shadow, bad.size, bad[:4])
+    finally:
+        ctx.set_tuning()

@@ -950,7 +950,11 @@ __device__ __forceinline__ void fetch_mnode(const MNode* mnodes, int node, unsig
 // ---- the octant walk of static nodes (ONode, device.h)
 // Two float32 operations in one instruction, each rounded as the scalar one
 // (add.rn / mul.rn .f32x2): the slab test's subtractions and products of two
-// axes at a time, and the three-operand min and max.
+// axes at a time, and the three-operand min and max.  No add2 takes a mul2's
+// result: the assembler (13.0.88) contracts that pair into a fused
+// multiply-add despite both .rn and -fmad=false (339,366 of 1,048,576 random
+// sums of products differed), so products that are added are scalar, which it
+// leaves alone.
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
   return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32);
 }
@@ -965,6 +969,10 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+// a * b + c * d per component, all three operations rounded.
+__device__ __forceinline__ uint64_t lerp2(float a, uint64_t b, float c, uint64_t d) {
+  return add2(pack2(__fmul_rn(a, lo2(b)), __fmul_rn(a, hi2(b))), pack2(__fmul_rn(c, lo2(d)), __fmul_rn(c, hi2(d))));
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
@@ -1026,9 +1034,9 @@ __device__ __forceinline__ void visit_octant(const ONode* p, const SlabRay& s, f
 
 // A motion node's octant copies of both keys (p0, p1: the same node of the
 // two keys), the planes lerped per float: (1.0-time)*Boxes[key] +
-// time*Boxes[key2] (motionintersect.go:47-49); tm2, omt2: the weights twice.
-__device__ __forceinline__ void visit_octant_m(const ONode* p0, const ONode* p1, const SlabRay& s, uint64_t tm2,
-                                               uint64_t omt2, float tclosest, Slots& o) {
+// time*Boxes[key2] (motionintersect.go:47-49).
+__device__ __forceinline__ void visit_octant_m(const ONode* p0, const ONode* p1, const SlabRay& s, float tm,
+                                               float omt, float tclosest, Slots& o) {
   const uint64_t* q0 = reinterpret_cast<const uint64_t*>(p0);
   const uint64_t* q1 = reinterpret_cast<const uint64_t*>(p1);
   uint64_t w[12];
@@ -1038,7 +1046,7 @@ __device__ __forceinline__ void visit_octant_m(const ONode* p0, const ONode* p1,
     ld_u64x4(q0 + 4 * k, a[0], a[1], a[2], a[3]);
     ld_u64x4(q1 + 4 * k, c[0], c[1], c[2], c[3]);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[4 * k + j] = add2(mul2(omt2, a[j]), mul2(tm2, c[j]));
+    for (int j = 0; j < 4; ++j) w[4 * k + j] = lerp2(omt, a[j], tm, c[j]);
   }
   const int4 c = __ldg(reinterpret_cast<const int4*>(p0->child));
   o.child[0] = c.x; o.child[1] = c.y; o.child[2] = c.z; o.child[3] = c.w;
@@ -1604,7 +1612,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
         if (obase < kNodesPlain) {
           Slots o;
           const ONode* on = m.onodes + (obase + (uint32_t)node);
-          if (MOTION) visit_octant_m(on, on + dkey, slab, pack2(tm, tm), pack2(omt, omt), r.tclosest, o);
+          if (MOTION) visit_octant_m(on, on + dkey, slab, tm, omt, r.tclosest, o);
           else visit_octant(on, slab, r.tclosest, o);
           pushed = push_slots(stk, sp, o, next, status);
         } else {
@@ -1934,7 +1942,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
               Slots o;
               if (MOT && level == kLevelMotion) {
                 const float omt = __fsub_rn(1.0f, tm);
-                visit_octant_m(on + node, on + node + dkey, slab, pack2(tm, tm), pack2(omt, omt), r.tclosest, o);
+                visit_octant_m(on + node, on + node + dkey, slab, tm, omt, r.tclosest, o);
               } else {
                 visit_octant(on + node, slab, r.tclosest, o);
               }
