@@ -185,6 +185,42 @@ __device__ __forceinline__ float kcomp(const TRay& r, const float4& v) {
   }
 }
 
+// Two float32 operations in one instruction, each rounded as the scalar one
+// (add.rn / mul.rn .f32x2): the slab test's and the watertight test's two axes at
+// a time, and the three-operand min and max.  x - y is x + (-y), and
+// (-s) * z is -(s * z).  No add2 takes a mul2's result: the assembler (13.0.88)
+// contracts that pair into a fused multiply-add despite both .rn and
+// -fmad=false (339,366 of 1,048,576 random sums of products differed), so
+// products that are added are scalar, which it leaves alone.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// a * b + c * d per component, all three operations rounded.
+__device__ __forceinline__ uint64_t lerp2(float a, uint64_t b, float c, uint64_t d) {
+  return add2(pack2(__fmul_rn(a, lo2(b)), __fmul_rn(a, hi2(b))), pack2(__fmul_rn(c, lo2(d)), __fmul_rn(c, hi2(d))));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // The watertight test (trace.go:123-193), in two parts.  tri_prepare: the
 // part that does not depend on Tclosest (edge functions with the FP64
 // fallback, the sign test, det, T and the lower bound); false when the
@@ -196,12 +232,12 @@ __device__ __forceinline__ bool tri_prepare(const TRay& r, float4 v0, float4 v1,
   const float AKz = __fsub_rn(kcomp<C, 2>(r, v0), r.pkz);
   const float BKz = __fsub_rn(kcomp<C, 2>(r, v1), r.pkz);
   const float CKz = __fsub_rn(kcomp<C, 2>(r, v2), r.pkz);
-  const float Cx = __fsub_rn(__fsub_rn(kcomp<C, 0>(r, v2), r.pkx), __fmul_rn(r.s0, CKz));
-  const float By = __fsub_rn(__fsub_rn(kcomp<C, 1>(r, v1), r.pky), __fmul_rn(r.s1, BKz));
-  const float Cy = __fsub_rn(__fsub_rn(kcomp<C, 1>(r, v2), r.pky), __fmul_rn(r.s1, CKz));
-  const float Bx = __fsub_rn(__fsub_rn(kcomp<C, 0>(r, v1), r.pkx), __fmul_rn(r.s0, BKz));
-  const float Ax = __fsub_rn(__fsub_rn(kcomp<C, 0>(r, v0), r.pkx), __fmul_rn(r.s0, AKz));
-  const float Ay = __fsub_rn(__fsub_rn(kcomp<C, 1>(r, v0), r.pky), __fmul_rn(r.s1, AKz));
+  const uint64_t np = pack2(-r.pkx, -r.pky);
+  const float n0 = -r.s0, n1 = -r.s1;
+  const uint64_t A2 = add2(add2(pack2(kcomp<C, 0>(r, v0), kcomp<C, 1>(r, v0)), np), pack2(__fmul_rn(n0, AKz), __fmul_rn(n1, AKz)));
+  const uint64_t B2 = add2(add2(pack2(kcomp<C, 0>(r, v1), kcomp<C, 1>(r, v1)), np), pack2(__fmul_rn(n0, BKz), __fmul_rn(n1, BKz)));
+  const uint64_t C2 = add2(add2(pack2(kcomp<C, 0>(r, v2), kcomp<C, 1>(r, v2)), np), pack2(__fmul_rn(n0, CKz), __fmul_rn(n1, CKz)));
+  const float Ax = lo2(A2), Ay = hi2(A2), Bx = lo2(B2), By = hi2(B2), Cx = lo2(C2), Cy = hi2(C2);
   fU = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
   fV = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
   fW = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
@@ -212,7 +248,7 @@ __device__ __forceinline__ bool tri_prepare(const TRay& r, float4 v0, float4 v1,
     fV = __double2float_rn(__dsub_rn(__dmul_rn((double)Ax, (double)Cy), __dmul_rn((double)Ay, (double)Cx)));
     fW = __double2float_rn(__dsub_rn(__dmul_rn((double)Bx, (double)Ay), __dmul_rn((double)By, (double)Ax)));
   }
-  if ((fU < 0.0f || fV < 0.0f || fW < 0.0f) && (fU > 0.0f || fV > 0.0f || fW > 0.0f)) return false;
+  if (min3(fU, fV, fW) < 0.0f && max3(fU, fV, fW) > 0.0f) return false;  // a NaN takes no side
   det = __fadd_rn(__fadd_rn(fU, fV), fW);
   if (det == 0.0f) return false;
   T = __fmul_rn(r.s2, __fadd_rn(__fadd_rn(__fmul_rn(fU, AKz), __fmul_rn(fV, BKz)), __fmul_rn(fW, CKz)));
@@ -947,43 +983,7 @@ __device__ __forceinline__ void fetch_mnode(const MNode* mnodes, int node, unsig
   rk = (((oct & 4u) ? meta.z : meta.y) >> ((oct & 3u) * 8u)) & 0xffu;
 }
 
-// ---- the octant walk of static nodes (ONode, device.h)
-// Two float32 operations in one instruction, each rounded as the scalar one
-// (add.rn / mul.rn .f32x2): the slab test's subtractions and products of two
-// axes at a time, and the three-operand min and max.  No add2 takes a mul2's
-// result: the assembler (13.0.88) contracts that pair into a fused
-// multiply-add despite both .rn and -fmad=false (339,366 of 1,048,576 random
-// sums of products differed), so products that are added are scalar, which it
-// leaves alone.
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32);
-}
-__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// a * b + c * d per component, all three operations rounded.
-__device__ __forceinline__ uint64_t lerp2(float a, uint64_t b, float c, uint64_t d) {
-  return add2(pack2(__fmul_rn(a, lo2(b)), __fmul_rn(a, hi2(b))), pack2(__fmul_rn(c, lo2(d)), __fmul_rn(c, hi2(d))));
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
+// ---- the octant walk of the nodes (ONode, device.h)
 __device__ __forceinline__ void ld_u64x4(const void* p, uint64_t& a, uint64_t& b, uint64_t& c, uint64_t& d) {
   asm("ld.global.nc.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
@@ -1297,9 +1297,27 @@ __device__ __forceinline__ int32_t leaf_scan_dispatch(const DMesh& m, TRay& r, u
 // sequential scan.  Called by all 32 lanes; has: the lane holds a leaf.
 // tris, lower: the lane's mesh (its triangles and lower bound); the tester
 // uses its owner's (one mesh per launch in the mesh kernel, one per lane in
-// the scene kernel).
+// the scene kernel).  map: the warp's 32 entries of one array in shared memory
+// (one a kernel: an array per instantiation costs L1 and measured slower than
+// the search it replaces).
+//
+// A position's leaf is the last one that starts at or before it: the round's
+// starts come from one warp reduction, the leaf's lane and triangle offset
+// from a table by the leaf's rank.  Against a five-step search by shuffle (whole
+// calls): 4,194,304 incoherent rays 6.28 -> 6.09 ms, 300,007 shadow rays 515 ->
+// 489 us, room render 5.73 -> 5.58 ms.
+__device__ __forceinline__ void locate_mapped(const int2* map, uint32_t base, uint32_t excl, bool has, int& o,
+                                              uint32_t& i) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t rel = excl - base;
+  const unsigned starts = __reduce_or_sync(kFull, has && rel < 32u ? 1u << rel : 0u);
+  const int before = __popc(__ballot_sync(kFull, has && excl < base)) - 1;
+  const int2 e = map[before + __popc(starts & (0xffffffffu >> (31u - lane)))];
+  o = e.x;
+  i = base + lane + (uint32_t)e.y;
+}
 template <int C>
-__device__ __forceinline__ int32_t coop_leaf(const float4* tris, float lower, TRay& r, bool has, uint32_t first,
+__device__ __forceinline__ int32_t coop_leaf(int2* map, const float4* tris, float lower, TRay& r, bool has, uint32_t first,
                                              uint32_t count, float& U, float& V, float& W) {
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t cnt = has ? count : 0u;
@@ -1311,19 +1329,15 @@ __device__ __forceinline__ int32_t coop_leaf(const float4* tris, float lower, TR
   }
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   const uint32_t excl = incl - cnt;
+  const unsigned hm = __ballot_sync(kFull, has);
+  if (has) map[__popc(hm & ((1u << lane) - 1u))] = make_int2((int)lane, (int)(first - excl));
+  __syncwarp();
   int32_t idx = -1;
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t g = base + lane;
-    // owner: the lowest lane whose inclusive prefix exceeds g
-    int lo = 0, hi = 31;
-#pragma unroll
-    for (int st = 0; st < 5; ++st) {
-      const int mid = (lo + hi) >> 1;
-      if (__shfl_sync(kFull, incl, mid) > g) hi = mid;
-      else lo = mid + 1;
-    }
-    const int o = lo;
-    const uint32_t i = __shfl_sync(kFull, first, o) + (g - __shfl_sync(kFull, excl, o));
+    int o;
+    uint32_t i;
+    locate_mapped(map, base, excl, has, o, i);
     TRay q;  // the owner's ray: the fields tri_prepare reads
     q.pkx = __shfl_sync(kFull, r.pkx, o);
     q.pky = __shfl_sync(kFull, r.pky, o);
@@ -1354,6 +1368,7 @@ __device__ __forceinline__ int32_t coop_leaf(const float4* tris, float lower, TR
       if ((int)lane == oc && tri_accept(r, cU, cV, cW, cdet, cT, U, V, W)) idx = (int32_t)ci;
     }
   }
+  __syncwarp();
   return idx;
 }
 
@@ -1363,10 +1378,13 @@ __device__ __forceinline__ int32_t coop_leaf(const float4* tris, float lower, TR
 // stored vertices above EpsilonFloat32 + RayBias; a motion pair is
 // TraceMotionElems' (trace.go:563-612) on the vertices of the two keys
 // lerped at the owner's time, Vec3Lerp (math/vec3.go:52-58), above RayBias.
-// Acceptance on the owner in triangle order, as in coop_leaf.  t1, tm, omt
+// Acceptance on the owner in triangle order, as in coop_leaf.  MAP: locate
+// positions as coop_leaf does (the mesh kernel: 262,147 rays on 100,000 moving
+// triangles 1.33 -> 1.30 ms); the scene kernel keeps the search (path jobs 6.30
+// against 6.38 ms).  t1, tm, omt
 // are unused by static owners.
-template <int C>
-__device__ __forceinline__ int32_t coop_leaf_mix(const float4* t0, const float4* t1, float tm, float omt, bool mot,
+template <int C, bool MAP>
+__device__ __forceinline__ int32_t coop_leaf_mix(int2* map, const float4* t0, const float4* t1, float tm, float omt, bool mot,
                                                  float lower, TRay& r, bool has, uint32_t first, uint32_t count,
                                                  float& U, float& V, float& W) {
   const unsigned lane = threadIdx.x & 31u;
@@ -1379,18 +1397,29 @@ __device__ __forceinline__ int32_t coop_leaf_mix(const float4* t0, const float4*
   }
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   const uint32_t excl = incl - cnt;
+  if (MAP) {
+    const unsigned hm = __ballot_sync(kFull, has);
+    if (has) map[__popc(hm & ((1u << lane) - 1u))] = make_int2((int)lane, (int)(first - excl));
+    __syncwarp();
+  }
   int32_t idx = -1;
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t g = base + lane;
-    int lo = 0, hi = 31;
+    int o;
+    uint32_t i;
+    if (MAP) {
+      locate_mapped(map, base, excl, has, o, i);
+    } else {
+      int lo = 0, hi = 31;
 #pragma unroll
-    for (int st = 0; st < 5; ++st) {
-      const int mid = (lo + hi) >> 1;
-      if (__shfl_sync(kFull, incl, mid) > g) hi = mid;
-      else lo = mid + 1;
+      for (int st = 0; st < 5; ++st) {
+        const int mid = (lo + hi) >> 1;
+        if (__shfl_sync(kFull, incl, mid) > g) hi = mid;
+        else lo = mid + 1;
+      }
+      o = lo;
+      i = __shfl_sync(kFull, first, o) + (g - __shfl_sync(kFull, excl, o));
     }
-    const int o = lo;
-    const uint32_t i = __shfl_sync(kFull, first, o) + (g - __shfl_sync(kFull, excl, o));
     TRay q;
     q.pkx = __shfl_sync(kFull, r.pkx, o);
     q.pky = __shfl_sync(kFull, r.pky, o);
@@ -1414,9 +1443,8 @@ __device__ __forceinline__ int32_t coop_leaf_mix(const float4* t0, const float4*
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const float4 a = __ldg(a0 + 3 * (size_t)i + j), c = __ldg(a1 + 3 * (size_t)i + j);
-          v[j] = make_float4(__fadd_rn(__fmul_rn(oomt, a.x), __fmul_rn(otm, c.x)),
-                             __fadd_rn(__fmul_rn(oomt, a.y), __fmul_rn(otm, c.y)),
-                             __fadd_rn(__fmul_rn(oomt, a.z), __fmul_rn(otm, c.z)), 0.f);
+          const uint64_t xy = lerp2(oomt, pack2(a.x, a.y), otm, pack2(c.x, c.y));
+          v[j] = make_float4(lo2(xy), hi2(xy), __fadd_rn(__fmul_rn(oomt, a.z), __fmul_rn(otm, c.z)), 0.f);
         }
         cand = tri_prepare<false, C>(q, v[0], v[1], v[2], olower, fU, fV, fW, det, T);
       } else {
@@ -1437,10 +1465,12 @@ __device__ __forceinline__ int32_t coop_leaf_mix(const float4* t0, const float4*
       if ((int)lane == oc && tri_accept(r, cU, cV, cW, cdet, cT, U, V, W)) idx = (int32_t)ci;
     }
   }
+  if (MAP) __syncwarp();
   return idx;
 }
 
-__device__ __forceinline__ int32_t coop_leaf_mix_dispatch(const float4* t0, const float4* t1, float tm, float omt,
+template <bool MAP>
+__device__ __forceinline__ int32_t coop_leaf_mix_dispatch(int2* map, const float4* t0, const float4* t1, float tm, float omt,
                                                           bool mot, float lower, TRay& r, bool has, uint32_t first,
                                                           uint32_t count, float& U, float& V, float& W) {
   const unsigned hm = __ballot_sync(kFull, has);
@@ -1448,35 +1478,35 @@ __device__ __forceinline__ int32_t coop_leaf_mix_dispatch(const float4* t0, cons
   const int c0 = __shfl_sync(kFull, r.cls, __ffs(hm) - 1);
   if (__all_sync(kFull, !has || r.cls == c0)) {
     switch (c0) {
-      case 0: return coop_leaf_mix<0>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
-      case 1: return coop_leaf_mix<1>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
-      case 2: return coop_leaf_mix<2>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
-      case 3: return coop_leaf_mix<3>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
-      case 4: return coop_leaf_mix<4>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
-      default: return coop_leaf_mix<5>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+      case 0: return coop_leaf_mix<0, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+      case 1: return coop_leaf_mix<1, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+      case 2: return coop_leaf_mix<2, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+      case 3: return coop_leaf_mix<3, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+      case 4: return coop_leaf_mix<4, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+      default: return coop_leaf_mix<5, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
     }
   }
-  return coop_leaf_mix<-1>(t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
+  return coop_leaf_mix<-1, MAP>(map, t0, t1, tm, omt, mot, lower, r, has, first, count, U, V, W);
 }
 
 // The class the lanes holding a leaf share picks the compile-time instance;
 // mixed classes take the run-time-select one.  All 32 lanes call this.
-__device__ __forceinline__ int32_t coop_leaf_dispatch(const float4* tris, float lower, TRay& r, bool has,
+__device__ __forceinline__ int32_t coop_leaf_dispatch(int2* map, const float4* tris, float lower, TRay& r, bool has,
                                                       uint32_t first, uint32_t count, float& U, float& V, float& W) {
   const unsigned hm = __ballot_sync(kFull, has);
   if (hm == 0u) return -1;
   const int c0 = __shfl_sync(kFull, r.cls, __ffs(hm) - 1);
   if (__all_sync(kFull, !has || r.cls == c0)) {
     switch (c0) {
-      case 0: return coop_leaf<0>(tris, lower, r, has, first, count, U, V, W);
-      case 1: return coop_leaf<1>(tris, lower, r, has, first, count, U, V, W);
-      case 2: return coop_leaf<2>(tris, lower, r, has, first, count, U, V, W);
-      case 3: return coop_leaf<3>(tris, lower, r, has, first, count, U, V, W);
-      case 4: return coop_leaf<4>(tris, lower, r, has, first, count, U, V, W);
-      default: return coop_leaf<5>(tris, lower, r, has, first, count, U, V, W);
+      case 0: return coop_leaf<0>(map, tris, lower, r, has, first, count, U, V, W);
+      case 1: return coop_leaf<1>(map, tris, lower, r, has, first, count, U, V, W);
+      case 2: return coop_leaf<2>(map, tris, lower, r, has, first, count, U, V, W);
+      case 3: return coop_leaf<3>(map, tris, lower, r, has, first, count, U, V, W);
+      case 4: return coop_leaf<4>(map, tris, lower, r, has, first, count, U, V, W);
+      default: return coop_leaf<5>(map, tris, lower, r, has, first, count, U, V, W);
     }
   }
-  return coop_leaf<-1>(tris, lower, r, has, first, count, U, V, W);
+  return coop_leaf<-1>(map, tris, lower, r, has, first, count, U, V, W);
 }
 
 template <bool MOTION, bool ANY, bool COUNT, bool PF, int MINB, int SS, bool COOP = false>
@@ -1485,6 +1515,8 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                     int walk_tail, const unsigned long long* n_dev) {
   if (n_dev) n = *n_dev < n ? *n_dev : n;  // a wavefront queue's length
   extern __shared__ int stack_smem[];
+  // a leaf phase's leaves of each warp by rank: lane, first triangle - first position
+  __shared__ int2 leaf_map[COOP ? (MINB > 0 ? 128 : 256) : 1];
   SplitStack<SS> stk;
   if (SS > 0) {
     stk.stride = blockDim.x;
@@ -1679,8 +1711,8 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
       float U = 0.f, V = 0.f, W = 0.f;
       // motion: every tester lerps its owner's two keys at the owner's time
       const int32_t idx =
-          MOTION ? coop_leaf_mix_dispatch(tr0, tr1, tm, omt, true, m.ray_bias, r, has, first, count, U, V, W)
-                 : coop_leaf_dispatch(reinterpret_cast<const float4*>(m.tris), m.lower_static, r, has, first, count,
+          MOTION ? coop_leaf_mix_dispatch<true>(leaf_map + (threadIdx.x & ~31u), tr0, tr1, tm, omt, true, m.ray_bias, r, has, first, count, U, V, W)
+                 : coop_leaf_dispatch(leaf_map + (threadIdx.x & ~31u), reinterpret_cast<const float4*>(m.tris), m.lower_static, r, has, first, count,
                                       U, V, W);
       if (has) {
         if (idx != -1) {
@@ -1755,6 +1787,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
     n = nd < n ? nd : n;
   }
   int2 stk[kStackCapacity];
+  __shared__ int2 leaf_map[128];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanes_below = (1u << lane) - 1u;
   TRay r;
@@ -2018,9 +2051,9 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
         }
       }
       if (COOP && MOT) {  // static and motion leaves in one cooperative list
-        idx = coop_leaf_mix_dispatch(t0, t1, lm, lomt, mot, lo, r, any_leaf, first, count, U, V, W);
+        idx = coop_leaf_mix_dispatch<false>(nullptr, t0, t1, lm, lomt, mot, lo, r, any_leaf, first, count, U, V, W);
       } else if (COOP) {
-        idx = coop_leaf_dispatch(t0, lo, r, any_leaf, first, count, U, V, W);
+        idx = coop_leaf_dispatch(leaf_map + (threadIdx.x & ~31u), t0, lo, r, any_leaf, first, count, U, V, W);
       } else if (any_leaf) {
         if (mot) {  // vertices lerped at the ray's time, scanned by its lane
           idx = leaf_scan_dispatch<true>(*M, r, first, count, t0, t1, lm, lomt, U, V, W);
