@@ -84,7 +84,8 @@ typedef struct {
                             5, a static leaf without it), 0..31 (default 8;
                             0 = wait for every lane) */
     int sort_bits;       /* sort-key width: the ray reordering groups origins
-                            in (2^b)^3 cells, b = 3, 4 or 5 (0: 4) */
+                            in (2^b)^3 cells, b = 3, 4 or 5 (0: 3 for
+                            batches below 700,000 rays, else 4) */
 } vmr_tuning;
 int vmr_set_tuning(vmr_ctx* ctx, const vmr_tuning* tuning);
 int vmr_get_tuning(vmr_ctx* ctx, vmr_tuning* tuning);

@@ -370,7 +370,7 @@ int launch_trace_chunk(vmr_ctx* ctx, const DMesh* mesh, const vmr_rays& r, size_
     // no ray times.
     const bool recs = mesh && mesh->keys <= 1 && (tn.kernel & vmr::kKernelWhileWhile);
     if (recs) sorted = vmr::RaySoA{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, order};
-    int se = vmr::launch_ray_sort(l.rays, n, mb, tn.sort_bits ? tn.sort_bits : 4, keys, hist, order, sorted,
+    int se = vmr::launch_ray_sort(l.rays, n, mb, tn.sort_bits ? tn.sort_bits : vmr::default_sort_bits(n), keys, hist, order, sorted,
                                   ctx->stream);
     if (se != 0) return cuda_fail(ctx, (cudaError_t)se, "ray sort launch");
     l.rays = sorted;

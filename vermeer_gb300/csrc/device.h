@@ -169,12 +169,16 @@ enum TraceKernel : int {
 constexpr int kSharedStackEntries = 16;
 
 // Ray reordering (raysort.cu): 6 permutation classes x (2^b)^3 origin cells,
-// b = 3..5 (default 4: 16^3 cells).
-constexpr int kSortCells = 4096;
-constexpr int kSortBuckets = 6 * kSortCells;
+// b = 3..5, x the octant of the class's other two signs for b <= 4.
 constexpr int kSortMaxBits = 5;
+constexpr int kSortOctantBits = 4;
 constexpr int kSortBucketsMax = 6 << (3 * kSortMaxBits);
-constexpr uint32_t sort_buckets(int bits) { return 6u << (3 * bits); }
+constexpr uint32_t sort_buckets(int bits) { return (6u << (3 * bits)) * (bits <= kSortOctantBits ? 4u : 1u); }
+// The width a tuning of 0 takes: 16^3 cells, or 8^3 for batches in which that
+// many buckets (98,304) would hold a few rays each and their scan costs more
+// than the finer cells give (300,007 rays: 488 against 495 us; 1,000,003: 460
+// against 456).
+constexpr int default_sort_bits(uint64_t n) { return n < 700000u ? 3 : 4; }
 constexpr uint64_t kSortMinRays = 1u << 16;  // smaller batches are traced unsorted
 
 // Launch entry points (traverse.cu).

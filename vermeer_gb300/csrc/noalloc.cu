@@ -161,7 +161,7 @@ extern "C" int vmr_trace_mesh_noalloc(vmr_ctx* ctx, uint32_t geom, const vmr_ray
     vmr::RaySoA sorted{f, f + kMaxRays, f + 2 * kMaxRays, f + 3 * kMaxRays, f + 4 * kMaxRays,
                        f + 5 * kMaxRays, f + 6 * kMaxRays, rays->time ? f + 7 * kMaxRays : nullptr};
     if (recs) sorted = vmr::RaySoA{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, f};
-    const int bits = tuning.sort_bits ? tuning.sort_bits : 4;
+    const int bits = tuning.sort_bits ? tuning.sort_bits : vmr::default_sort_bits(n);
     if (bits > vmr::kSortMaxBits)
       return vmr::ctx_fail(ctx, VMR_ERR_INVALID, "vmr_trace_mesh_noalloc: sort key wider than the histogram");
     if (vmr::launch_ray_sort(l.rays, n, bounds, bits, keys, hist, order, sorted, stream) != 0)
