@@ -202,12 +202,13 @@ __device__ __forceinline__ void sincos_turns(float u, float& s, float& c) {
 }
 
 // ----------------------------------------------------------- material ----
+// The weights and roughnesses; colours and Fresnel parameters are read from
+// the shader where they are used (a lane would hold them across the vertex).
 struct Mat {
   float dw, sw;
-  V3 cd, cs;
   float rd, alpha;
   bool mirror;
-  Fresnel fr;
+  const vmr_shader_std* sh;
 };
 
 __device__ __forceinline__ Mat material(const vmr_shader_std& s) {
@@ -217,22 +218,30 @@ __device__ __forceinline__ Mat material(const vmr_shader_std& s) {
   const float tw = dw + sw;
   m.dw = dw / tw;
   m.sw = sw / tw;
-  m.cd = (s.flags & VMR_SH_DIFFUSE_COLOUR) ? v3(s.diffuse_colour[0], s.diffuse_colour[1], s.diffuse_colour[2])
-                                           : v3(0, 0, 0);
-  m.cs = (s.flags & VMR_SH_SPEC1_COLOUR) ? v3(s.spec1_colour[0], s.spec1_colour[1], s.spec1_colour[2]) : v3(0, 0, 0);
   m.rd = (s.flags & VMR_SH_DIFFUSE_ROUGHNESS) ? s.diffuse_roughness : 0.5f;
   const float rs = (s.flags & VMR_SH_SPEC1_ROUGHNESS) ? s.spec1_roughness : 0.5f;
   m.mirror = rs == 0.0f;
   m.alpha = sqr(rs * rs);
-  m.fr = Fresnel{0, (s.flags & VMR_SH_IOR) ? s.ior : 1.7f, {}, {}};
+  m.sh = &s;
+  return m;
+}
+__device__ __forceinline__ V3 diffuse_colour(const vmr_shader_std& s) {
+  return (s.flags & VMR_SH_DIFFUSE_COLOUR) ? v3(s.diffuse_colour[0], s.diffuse_colour[1], s.diffuse_colour[2])
+                                           : v3(0, 0, 0);
+}
+__device__ __forceinline__ V3 spec1_colour(const vmr_shader_std& s) {
+  return (s.flags & VMR_SH_SPEC1_COLOUR) ? v3(s.spec1_colour[0], s.spec1_colour[1], s.spec1_colour[2]) : v3(0, 0, 0);
+}
+__device__ __forceinline__ RGB spec1_kr(const vmr_shader_std& s, float c) {
+  Fresnel fr{0, (s.flags & VMR_SH_IOR) ? s.ior : 1.7f, {}, {}};
   if (s.spec1_fresnel == 1) {
     RGB refl{{0.5f, 0.5f, 0.5f}}, edge{{0.5f, 0.5f, 0.5f}};
     if (s.flags & VMR_SH_FRESNEL_REFL) refl = RGB{{s.spec1_fresnel_refl[0], s.spec1_fresnel_refl[1], s.spec1_fresnel_refl[2]}};
     if (s.flags & VMR_SH_FRESNEL_EDGE)  // the reference's assignment (std.go:185-187)
       refl = RGB{{s.spec1_fresnel_edge[0], s.spec1_fresnel_edge[1], s.spec1_fresnel_edge[2]}};
-    m.fr = Fresnel{1, 0, refl, edge};
+    fr = Fresnel{1, 0, refl, edge};
   }
-  return m;
+  return fresnel_kr(fr, c);
 }
 
 __device__ __forceinline__ float ggx_d_pt(V3 m, float alpha) {
@@ -242,14 +251,18 @@ __device__ __forceinline__ float ggx_d_pt(V3 m, float alpha) {
   return (alpha * alpha) / denom;
 }
 
-// f(wi, wo)*|cos wo| in the local frame (wi.z > 0: the frame faces wi).
-__device__ V3 bsdf_f(const Mat& m, V3 wi, V3 wo) {
-  V3 f = v3(0, 0, 0);
-  if (wo.z <= 0.0f) return f;
+// f(wi, wo)*|cos wo| in the local frame (wi.z > 0: the frame faces wi) and the
+// density p the BSDF samples wo with.  Both need the half vector and the
+// distribution at it, so they are evaluated together.
+__device__ __forceinline__ void bsdf_f_pdf(const Mat& m, V3 wi, V3 wo, V3& f, float& p) {
+  f = v3(0, 0, 0);
+  p = 0.0f;
+  if (wo.z <= 0.0f) return;
+  const float lambert = wo.z / kPi;
   if (m.dw > 0.0f) {
     float s;
     if (m.rd == 0.0f) {
-      s = wo.z / kPi;
+      s = lambert;
     } else {  // OrenNayar (bsdf/orennayar.go:42-73), sigma = roughness^2
       // without angles: alpha = max(theta), beta = min(theta) of the two
       // directions, so sin(alpha) = sin(theta) of the smaller cos and
@@ -266,30 +279,24 @@ __device__ V3 bsdf_f(const Mat& m, V3 wi, V3 wo) {
       s = wo.z * (A + (B * (gm > 0.0f ? gm : 0.0f) * C)) / kPi;
     }
     const float k = m.dw * s;
-    f = v3(k * m.cd.x, k * m.cd.y, k * m.cd.z);
+    const V3 cd = diffuse_colour(*m.sh);
+    f = v3(k * cd.x, k * cd.y, k * cd.z);
   }
+  p = m.dw * lambert;
   if (m.sw > 0.0f && !m.mirror) {
     const V3 h = normalize(add(wi, wo));
-    const RGB F = fresnel_kr(m.fr, fabsf(dot(wi, h)));
-    const float numer = ggx_g1(wi, h, m.alpha) * ggx_g1(wo, h, m.alpha) * ggx_d_pt(h, m.alpha);
+    const RGB F = spec1_kr(*m.sh, fabsf(dot(wi, h)));
+    const V3 cs = spec1_colour(*m.sh);
+    const float D = ggx_d_pt(h, m.alpha);
+    const float numer = ggx_g1(wi, h, m.alpha) * ggx_g1(wo, h, m.alpha) * D;
     const float denom = 4 * wi.z * wo.z;
     float s = wo.z * numer / denom;
     if (!(s > 0.0f)) s = 0.0f;
     const float k = m.sw * s;
-    f = add(f, v3(k * m.cs.x * F.c[0], k * m.cs.y * F.c[1], k * m.cs.z * F.c[2]));
-  }
-  return f;
-}
-
-__device__ float bsdf_pdf_pt(const Mat& m, V3 wi, V3 wo) {
-  if (wo.z <= 0.0f) return 0.0f;
-  float p = m.dw * (wo.z / kPi);
-  if (m.sw > 0.0f && !m.mirror) {
-    const V3 h = normalize(add(wi, wo));
+    f = add(f, v3(k * cs.x * F.c[0], k * cs.y * F.c[1], k * cs.z * F.c[2]));
     const float d = fabsf(dot(wo, h));
-    if (d > 0.0f) p = p + m.sw * (ggx_d_pt(h, m.alpha) * h.z / (4 * d));
+    if (d > 0.0f) p = p + m.sw * (D * h.z / (4 * d));
   }
-  return p;
 }
 
 __device__ __forceinline__ float power_w(float a, float b) { return (a * a) / (a * a + b * b); }
@@ -454,12 +461,31 @@ __global__ void __launch_bounds__(kPtBlock) k_pt_prep(PtBatch b, uint32_t d) {
 // (probability alpha) and the BSDF at non-mirror vertices; TRAIN: training
 // records of the guided continuations; GROUPS: the scene has GeomInstances,
 // Procs or keyed mesh transforms (their transforms applied at each hit).
-// Registers capped for 3 resident blocks per SM (2 guided): measured faster
-// than the uncapped 121 (166) registers despite a few spilled words; the
-// GROUPS instantiation, which holds the keyed-transform helpers' registers,
-// is left uncapped.
-template <bool GUIDED, bool TRAIN, bool GROUPS>
-__global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : 3)) k_pt_shade(PtBatch b, uint32_t d) {
+// The GROUPS instantiation, which holds the keyed-transform helpers' registers,
+// is left uncapped; GUIDED is capped for 2 resident blocks per SM.
+//
+// What bounded it was instruction fetch: written as one nest of branches, the
+// lanes of a warp (different lights, lobes, materials) came back together
+// only at its end, at 8.9 of 32 lanes active, through two copies of the BSDF;
+// 8.7 of 16 stall cycles an issue were missing instructions and DRAM ran at 9%.
+// So the vertex is a sequence of short phases, the warp together again after
+// each, and the BSDF one piece of code both directions go through.
+//
+// BIG (batches of kPtBigBatch paths or more): a block's warps also wait for each
+// other between phases, so they fetch a phase's instructions once for all, at
+// 4 blocks per SM (64 registers); the sphere grid's 8.3M-path render 11.39 ->
+// 10.72 ms (warps alone 11.28 at 3 blocks, 11.10 at 4).  In a smaller batch a
+// warp waits mostly on its own chain: warps alone at 3 blocks (80 registers),
+// both directions' BSDF inline: 3,072 paths 576 us (590 with BIG), 16 jobs of
+// 131,072 paths 6.32 ms (6.34).
+constexpr uint64_t kPtBigBatch = 1u << 22;
+template <bool BIG>
+__device__ __forceinline__ void phase_end() {
+  if (BIG) __syncthreads();
+  else __syncwarp();
+}
+template <bool GUIDED, bool TRAIN, bool GROUPS, bool BIG = false>
+__global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : (BIG ? 4 : 3))) k_pt_shade(PtBatch b, uint32_t d) {
   const uint64_t n = b.qlen[d] < b.cap ? b.qlen[d] : b.cap;
   const float* q = b.qray[d & 1];
   const uint32_t* qp = b.qpath[d & 1];
@@ -470,23 +496,20 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : 3)) k_pt_
   // warp-aggregated appends see whole warps.
   const uint64_t nround = (n + stride - 1) / stride;
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const int nL = (int)b.nl;
+  const uint32_t base = 8 * d;
   for (uint64_t r = 0; r < nround; ++r) {
     const uint64_t i = r * stride + tid;
-    const bool active = i < n;
-    bool want_shadow = false, want_next = false;
-    uint32_t p = 0;
-    float so[3] = {0, 0, 0}, no[3] = {0, 0, 0};
-    V3 sd = v3(0, 0, 0), nd = v3(0, 0, 0), sc3 = v3(0, 0, 0);
-    float stmax = 0.f, time = 0.f;
-    bool want_rec = false;
-    V3 rP = v3(0, 0, 0), rN = v3(0, 0, 0), rWi = v3(0, 0, 0);
-    float rQ = 0.f, rPb = 0.f;
-    float nee_w = 0.f, nee_pb = 0.f;  // TRAIN: the light sample's record weight, BSDF density
-    if (active) {
+    uint32_t p = 0, shid = 0;
+    uint64_t key = 0;
+    bool shade = false;  // the vertex scatters: light sample and continuation
+    V3 beta = v3(0, 0, 0), wi = v3(0, 0, 0), org = v3(0, 0, 0);
+    Ctx sc;
+    // ---- the hit: attributes, emission or environment with MIS
+    if (i < n) {
       p = qp[i];
       const V3 D = v3(q[3 * (size_t)b.cap + i], q[4 * (size_t)b.cap + i], q[5 * (size_t)b.cap + i]);
-      time = q[7 * (size_t)b.cap + i];
-      V3 beta = v3(b.bx[p], b.by[p], b.bz[p]);
+      beta = v3(b.bx[p], b.by[p], b.bz[p]);
       V3 L = v3(b.lx[p], b.ly[p], b.lz[p]);
       if (TRAIN) {  // the radiance before this vertex closes the previous record
         const uint32_t lr = b.last_rec[p];
@@ -498,27 +521,29 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : 3)) k_pt_
         }
       }
       const float pdf_prev = b.pdf[p];
-      const uint64_t key = b.key[p];
+      key = b.key[p];
       const int32_t prim = b.hprim[i];
-      bool cont = false;
+      V3 Le = v3(0, 0, 0);
+      float w = 1.0f;  // the MIS weight of what the ray found by itself
+      bool emits = false;
       if (prim < 0) {
         if (b.has_env) {
-          const float w = pdf_prev == 0.0f ? 1.0f : power_w(pdf_prev, b.sel * kInv4Pi);
-          L = add(L, v3(beta.x * b.env[0] * w, beta.y * b.env[1] * w, beta.z * b.env[2] * w));
+          emits = true;
+          Le = v3(b.env[0], b.env[1], b.env[2]);
+          if (pdf_prev != 0.0f) w = power_w(pdf_prev, b.sel * kInv4Pi);
         }
       } else {
         const int32_t geom = b.hgeom[i];
-        Ctx sc;
-        uint32_t shid = 0;
         const V3 Ro = v3(q[i], q[(size_t)b.cap + i], q[2 * (size_t)b.cap + i]);
-        if (surface_attributes<GROUPS>(b.meshes[geom], prim, b.hu[i], b.hv[i], b.hw[i], Ro, D, b.ht[i], time, sc, shid)) {
+        if (surface_attributes<GROUPS>(b.meshes[geom], prim, b.hu[i], b.hv[i], b.hw[i], Ro, D, b.ht[i],
+                                       q[7 * (size_t)b.cap + i], sc, shid)) {
           const vmr_shader_std& sh = b.shaders[shid];
-          const V3 wi = v3(-D.x, -D.y, -D.z);
+          wi = v3(-D.x, -D.y, -D.z);
           const bool front = dot(sc.Ng, wi) > 0.0f;
           const RGB e = emission(sh);
-          const V3 Le = v3(e.c[0], e.c[1], e.c[2]);
+          Le = v3(e.c[0], e.c[1], e.c[2]);
           if (front && (Le.x != 0.0f || Le.y != 0.0f || Le.z != 0.0f)) {
-            float w = 1.0f;
+            emits = true;
             const int32_t li = (uint32_t)geom < b.n_geoms ? b.light_of_geom[geom] : -1;
             if (pdf_prev != 0.0f && li >= 0) {
               const PtLight& l = b.lights[li];
@@ -526,193 +551,199 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : 3)) k_pt_
               const float pl = b.sel * (t * t) / (l.area * fabsf(dot(D, sc.Ng)));
               w = power_w(pdf_prev, pl);
             }
-            L = add(L, v3(beta.x * Le.x * w, beta.y * Le.y * w, beta.z * Le.z * w));
           }
           const float tw = ((sh.flags & VMR_SH_DIFFUSE_STRENGTH) ? sh.diffuse_strength : 0.0f) +
                            ((sh.flags & VMR_SH_SPEC1_STRENGTH) ? sh.spec1_strength : 0.0f);
-          if (d < b.max_depth && tw != 0.0f) {
-            if (!front) {  // two-sided: face the incoming ray
-              sc.N = v3(-sc.N.x, -sc.N.y, -sc.N.z);
-              sc.Ng = v3(-sc.Ng.x, -sc.Ng.y, -sc.Ng.z);
-              sc.Poffset = v3(-sc.Poffset.x, -sc.Poffset.y, -sc.Poffset.z);
-            }
-            V3 Vt = cross(sc.N, sc.DdPdu);
-            if (len2(Vt) < 0.1f) Vt = cross(sc.N, sc.DdPdv);
-            Vt = normalize(Vt);
-            const V3 Ut = normalize(cross(sc.N, Vt));
-            const Mat m = material(sh);
-            const V3 wil = project(Ut, Vt, sc.N, wi);
-            const uint32_t base = 8 * d;
-            const int nL = (int)b.nl;
-            const bool guided = GUIDED && (m.dw > 0.0f || !m.mirror);
-            GMix gm;
-            if (guided) gmix_decode(b.gout + i * guide::kGuideOutStride, b.alpha, b.learn_sel != 0, gm);
-            // ---- next-event estimation
-            if (nL > 0 && (m.dw > 0.0f || !m.mirror)) {
-              const float u = rnd(key, base + 0);
-              int li = (int)(u * (float)nL);
-              if (li > nL - 1) li = nL - 1;
-              const float u0 = rnd(key, base + 1), u1 = rnd(key, base + 2);
-              const PtLight& l = b.lights[li];
-              V3 Ld;
-              float dist = 0.f, pl = 0.f;
-              bool ok = true;
-              if (l.kind == 2) {
-                const float z = 1 - 2 * u0;
-                const float rr = sqrtf((1 - z * z) > 0.0f ? (1 - z * z) : 0.0f);
-                float sp, cp;
-                sincos_turns(u1, sp, cp);
-                Ld = v3(rr * cp, rr * sp, z);
-                pl = b.sel * kInv4Pi;
-              } else {
-                const V3 p0 = v3(l.p0[0], l.p0[1], l.p0[2]), la = v3(l.a[0], l.a[1], l.a[2]),
-                         lb = v3(l.b[0], l.b[1], l.b[2]);
-                V3 Pl;
-                if (l.kind == 0) {
-                  const float su = sqrtf(u0);
-                  const float b0 = 1 - su, b1 = su * (1 - u1), b2 = su * u1;
-                  Pl = add(add(scale(b0, p0), scale(b1, la)), scale(b2, lb));
-                } else {
-                  Pl = add(add(p0, scale(u0, la)), scale(u1, lb));
-                }
-                const V3 Dv = sub(Pl, sc.P);
-                dist = length(Dv);
-                Ld = normalize(Dv);
-                const float cl = dot(Ld, v3(l.N[0], l.N[1], l.N[2]));
-                if (!(cl < 0.0f)) ok = false;
-                else pl = b.sel * (dist * dist) / (l.area * (-cl));
-              }
-              if (ok && dot(Ld, sc.Ng) > 0.0f && dot(Ld, sc.N) > 0.0f && pl > 0.0f && !isinf(pl)) {
-                const V3 wol = project(Ut, Vt, sc.N, Ld);
-                const V3 f = bsdf_f(m, wil, wol);
-                const float pbs = bsdf_pdf_pt(m, wil, wol);
-                const float pb = guided ? gm.alpha * gmix_pdf(gm, Ld) + (1.0f - gm.alpha) * pbs : pbs;
-                const float w = power_w(pl, pb);
-                const float k = w / pl;
-                const V3 c = v3(beta.x * f.x * l.Le[0] * k, beta.y * f.y * l.Le[1] * k, beta.z * f.z * l.Le[2] * k);
-                if (c.x > 0.0f || c.y > 0.0f || c.z > 0.0f) {
-                  const V3 o = offset_p(sc, 1);
-                  so[0] = o.x; so[1] = o.y; so[2] = o.z;
-                  if (l.kind == 2) {
-                    sd = Ld;
-                    stmax = __int_as_float(0x7f800000);
-                  } else {
-                    const float sl = dist * 0.9999f;
-                    sd = v3(Ld.x * sl, Ld.y * sl, Ld.z * sl);
-                    stmax = 1.0f;
-                  }
-                  sc3 = c;
-                  want_shadow = true;
-                  if (TRAIN && guided) {
-                    // incident radiance x |cos| over the light's density, with
-                    // the light's MIS weight: summed with the continuation
-                    // records (whose emission carries the other weight) it
-                    // estimates the product the guide is fitted to
-                    const float lum = 0.2126f * l.Le[0] + 0.7152f * l.Le[1] + 0.0722f * l.Le[2];
-                    const float wt = lum * w * fabsf(dot(sc.N, Ld)) / pl;
-                    nee_w = isfinite(wt) ? fminf(wt, 1e4f) : 0.f;
-                    rN = sc.N;
-                    rWi = wi;
-                    nee_pb = pbs;
-                  }
-                }
-              }
-            }
-            // ---- continuation: the guide (probability alpha) or the BSDF
-            const float ul = rnd(key, base + 3);
-            const float r0 = rnd(key, base + 4), r1 = rnd(key, base + 5);
-            V3 wol, wo;
-            bool delta = false;
-            const bool from_guide = guided && rnd(key, base + 7) < gm.alpha;
-            if (from_guide) {
-              wo = gmix_sample(gm, ul, r0, r1);
-              wol = project(Ut, Vt, sc.N, wo);
-            } else if (ul < m.dw) {  // CosineHemisphere (math/sample/sample.go:18-27), float32
-              const float r = sqrtf(1.0f - r0);
-              float sp, cp;
-              sincos_turns(r1, sp, cp);
-              wol = v3(r * cp, r * sp, sqrtf(r0));
-            } else if (m.mirror) {
-              wol = v3(-wil.x, -wil.y, wil.z);
-              delta = true;
-            } else {  // GGX D(m)cos(m) (microfacetggx.go:82-100): tan(theta_m) = alpha sqrt(r0) / sqrt(1-r0)
-              const float a = m.alpha * sqrtf(r0), bq = sqrtf(1.0f - r0);
-              const float hyp = sqrtf(a * a + bq * bq);
-              const float st = a / hyp, ct = bq / hyp;
-              float sp, cp;
-              sincos_turns(r1, sp, cp);
-              const V3 mh = v3(st * cp, st * sp, ct);
-              wol = normalize(sub(scale(2 * fabsf(dot(mh, wil)), mh), wil));
-            }
-            if (!from_guide) wo = expand(Ut, Vt, sc.N, wol);
-            if (dot(wo, sc.Ng) > 0.0f) {
-              bool alive = true;
-              float pb = 0.0f;
-              if (delta) {
-                const RGB F = fresnel_kr(m.fr, wil.z);
-                beta = v3(beta.x * (m.cs.x * F.c[0]), beta.y * (m.cs.y * F.c[1]), beta.z * (m.cs.z * F.c[2]));
-                if (guided) {  // the mirror lobe is taken with probability (1-alpha)*sw
-                  const float inv = 1.0f / (1.0f - gm.alpha);
-                  beta = v3(beta.x * inv, beta.y * inv, beta.z * inv);
-                }
-              } else {
-                const V3 f = bsdf_f(m, wil, wol);
-                pb = bsdf_pdf_pt(m, wil, wol);
-                rPb = pb;
-                if (guided) pb = gm.alpha * gmix_pdf(gm, wo) + (1.0f - gm.alpha) * pb;
-                if (!(pb > 0.0f)) alive = false;
-                else beta = v3(beta.x * (f.x / pb), beta.y * (f.y / pb), beta.z * (f.z / pb));
-              }
-              if (alive && d + 1 >= b.rr_depth) {  // Russian roulette
-                float qq = tmax3(beta.x, beta.y, beta.z);
-                if (qq > 0.95f) qq = 0.95f;
-                const float ur = rnd(key, base + 6);
-                if (!(ur < qq)) alive = false;
-                else beta = v3(beta.x / qq, beta.y / qq, beta.z / qq);
-              }
-              if (alive) {
-                const V3 o = offset_p(sc, 1);
-                no[0] = o.x; no[1] = o.y; no[2] = o.z;
-                nd = wo;
-                b.pdf[p] = delta ? 0.0f : pb;
-                cont = true;
-                if (TRAIN && guided && !delta) {
-                  want_rec = true;
-                  rP = sc.P;
-                  rN = sc.N;
-                  rWi = wi;
-                  rQ = pb;
-                }
-              }
-            }
+          shade = d < b.max_depth && tw != 0.0f;
+          if (!front) {  // two-sided: face the incoming ray
+            sc.N = v3(-sc.N.x, -sc.N.y, -sc.N.z);
+            sc.Ng = v3(-sc.Ng.x, -sc.Ng.y, -sc.Ng.z);
+            sc.Poffset = v3(-sc.Poffset.x, -sc.Poffset.y, -sc.Poffset.z);
           }
         }
       }
+      if (emits) L = add(L, v3(beta.x * Le.x * w, beta.y * Le.y * w, beta.z * Le.z * w));
       b.lx[p] = L.x; b.ly[p] = L.y; b.lz[p] = L.z;
-      if (cont) {
-        b.bx[p] = beta.x; b.by[p] = beta.y; b.bz[p] = beta.z;
-        want_next = true;
-      }
     }
-    __syncwarp();
+    phase_end<BIG>();
+    // ---- the shading frame and the material
+    Mat m{};
+    V3 Ut = v3(0, 0, 0), Vt = v3(0, 0, 0), wil = v3(0, 0, 0);
+    GMix gm;
+    bool guided = false;
+    if (shade) {
+      org = offset_p(sc, 1);
+      Vt = cross(sc.N, sc.DdPdu);
+      if (len2(Vt) < 0.1f) Vt = cross(sc.N, sc.DdPdv);
+      Vt = normalize(Vt);
+      Ut = normalize(cross(sc.N, Vt));
+      m = material(b.shaders[shid]);
+      wil = project(Ut, Vt, sc.N, wi);
+      guided = GUIDED && (m.dw > 0.0f || !m.mirror);
+      if (guided) gmix_decode(b.gout + i * guide::kGuideOutStride, b.alpha, b.learn_sel != 0, gm);
+    }
+    phase_end<BIG>();
+    // ---- next-event estimation: one light, its direction and density
+    bool nee = shade && nL > 0 && (m.dw > 0.0f || !m.mirror);
+    const PtLight* l = b.lights;
+    V3 Ld = v3(0, 0, 0);
+    float dist = 0.f, pl = 0.f;
+    if (nee) {
+      int li = (int)(rnd(key, base + 0) * (float)nL);
+      if (li > nL - 1) li = nL - 1;
+      l = b.lights + li;
+      const float u0 = rnd(key, base + 1), u1 = rnd(key, base + 2);
+      if (l->kind == 2) {
+        const float z = 1 - 2 * u0;
+        const float rr = sqrtf((1 - z * z) > 0.0f ? (1 - z * z) : 0.0f);
+        float sp, cp;
+        sincos_turns(u1, sp, cp);
+        Ld = v3(rr * cp, rr * sp, z);
+        pl = b.sel * kInv4Pi;
+      } else {
+        const V3 p0 = v3(l->p0[0], l->p0[1], l->p0[2]), la = v3(l->a[0], l->a[1], l->a[2]),
+                 lb = v3(l->b[0], l->b[1], l->b[2]);
+        V3 Pl;
+        if (l->kind == 0) {
+          const float su = sqrtf(u0);
+          const float b0 = 1 - su, b1 = su * (1 - u1), b2 = su * u1;
+          Pl = add(add(scale(b0, p0), scale(b1, la)), scale(b2, lb));
+        } else {
+          Pl = add(add(p0, scale(u0, la)), scale(u1, lb));
+        }
+        const V3 Dv = sub(Pl, sc.P);
+        dist = length(Dv);
+        Ld = normalize(Dv);
+        const float cl = dot(Ld, v3(l->N[0], l->N[1], l->N[2]));
+        if (!(cl < 0.0f)) nee = false;
+        else pl = b.sel * (dist * dist) / (l->area * (-cl));
+      }
+      nee = nee && dot(Ld, sc.Ng) > 0.0f && dot(Ld, sc.N) > 0.0f && pl > 0.0f && !isinf(pl);
+    }
+    phase_end<BIG>();
+    // ---- continuation: a direction from the guide (probability alpha) or
+    // the BSDF
+    V3 wo = v3(0, 0, 0), wol = v3(0, 0, 0);
+    bool delta = false, cont = false;
+    if (shade) {
+      const float ul = rnd(key, base + 3);
+      const float r0 = rnd(key, base + 4), r1 = rnd(key, base + 5);
+      const bool from_guide = guided && rnd(key, base + 7) < gm.alpha;
+      if (from_guide) {
+        wo = gmix_sample(gm, ul, r0, r1);
+        wol = project(Ut, Vt, sc.N, wo);
+      } else {
+        float sp, cp;
+        sincos_turns(r1, sp, cp);
+        if (ul < m.dw) {  // CosineHemisphere (math/sample/sample.go:18-27), float32
+          const float rr = sqrtf(1.0f - r0);
+          wol = v3(rr * cp, rr * sp, sqrtf(r0));
+        } else if (m.mirror) {
+          wol = v3(-wil.x, -wil.y, wil.z);
+          delta = true;
+        } else {  // GGX D(m)cos(m) (microfacetggx.go:82-100): tan(theta_m) = alpha sqrt(r0) / sqrt(1-r0)
+          const float a = m.alpha * sqrtf(r0), bq = sqrtf(1.0f - r0);
+          const float hyp = sqrtf(a * a + bq * bq);
+          const float st = a / hyp, ct = bq / hyp;
+          const V3 mh = v3(st * cp, st * sp, ct);
+          wol = normalize(sub(scale(2 * fabsf(dot(mh, wil)), mh), wil));
+        }
+        wo = expand(Ut, Vt, sc.N, wol);
+      }
+      cont = dot(wo, sc.Ng) > 0.0f;
+    }
+    phase_end<BIG>();
+    // ---- the BSDF toward the light, then along the continuation
+    bool want_shadow = false, want_rec = false;
+    V3 sc3 = v3(0, 0, 0);
+    float rQ = 0.f, rPb = 0.f;
+    float nee_w = 0.f, nee_pb = 0.f;  // TRAIN: the light sample's record weight, BSDF density
+#pragma unroll(BIG ? 1 : 2)
+    for (int pass = 0; pass < 2; ++pass) {
+      const bool on = pass == 0 ? nee : cont && !delta;
+      V3 f;
+      float pbs = 0.f, pb = 0.f;
+      if (on) {
+        const V3 w = pass == 0 ? Ld : wo;
+        bsdf_f_pdf(m, wil, pass == 0 ? project(Ut, Vt, sc.N, Ld) : wol, f, pbs);
+        pb = guided ? gm.alpha * gmix_pdf(gm, w) + (1.0f - gm.alpha) * pbs : pbs;
+      }
+      phase_end<BIG>();
+      if (pass == 0) {
+        if (nee) {
+          const float w = power_w(pl, pb);
+          const float k = w / pl;
+          const V3 c = v3(beta.x * f.x * l->Le[0] * k, beta.y * f.y * l->Le[1] * k, beta.z * f.z * l->Le[2] * k);
+          if (c.x > 0.0f || c.y > 0.0f || c.z > 0.0f) {
+            sc3 = c;
+            want_shadow = true;
+            if (TRAIN && guided) {
+              // incident radiance x |cos| over the light's density, with
+              // the light's MIS weight: summed with the continuation
+              // records (whose emission carries the other weight) it
+              // estimates the product the guide is fitted to
+              const float lum = 0.2126f * l->Le[0] + 0.7152f * l->Le[1] + 0.0722f * l->Le[2];
+              const float wt = lum * w * fabsf(dot(sc.N, Ld)) / pl;
+              nee_w = isfinite(wt) ? fminf(wt, 1e4f) : 0.f;
+              nee_pb = pbs;
+            }
+          }
+        }
+      } else if (cont) {
+        if (delta) {
+          const RGB F = spec1_kr(*m.sh, wil.z);
+          const V3 cs = spec1_colour(*m.sh);
+          beta = v3(beta.x * (cs.x * F.c[0]), beta.y * (cs.y * F.c[1]), beta.z * (cs.z * F.c[2]));
+          if (guided) {  // the mirror lobe is taken with probability (1-alpha)*sw
+            const float inv = 1.0f / (1.0f - gm.alpha);
+            beta = v3(beta.x * inv, beta.y * inv, beta.z * inv);
+          }
+        } else if (pb > 0.0f) {
+          beta = v3(beta.x * (f.x / pb), beta.y * (f.y / pb), beta.z * (f.z / pb));
+          rPb = pbs;
+          rQ = pb;
+        } else {
+          cont = false;
+        }
+        if (cont && d + 1 >= b.rr_depth) {  // Russian roulette
+          float qq = tmax3(beta.x, beta.y, beta.z);
+          if (qq > 0.95f) qq = 0.95f;
+          const float ur = rnd(key, base + 6);
+          if (!(ur < qq)) cont = false;
+          else beta = v3(beta.x / qq, beta.y / qq, beta.z / qq);
+        }
+        want_rec = TRAIN && cont && guided && !delta;
+      }
+      phase_end<BIG>();
+    }
+    const float so[3] = {org.x, org.y, org.z};
+    const float time = i < n ? q[7 * (size_t)b.cap + i] : 0.0f;
+    if (cont) {
+      b.pdf[p] = delta ? 0.0f : rQ;
+      b.bx[p] = beta.x; b.by[p] = beta.y; b.bz[p] = beta.z;
+    }
+    phase_end<BIG>();
     const unsigned long long si = warp_append(&b.slen[d], want_shadow);
     if (want_shadow && si < b.cap) {
-      put_ray(b.sray, b.cap, si, so, sd, stmax, time);
+      const float sl = dist * 0.9999f;  // a light's point at t = 1; the environment at infinity
+      const bool far = l->kind == 2;
+      put_ray(b.sray, b.cap, si, so, far ? Ld : v3(Ld.x * sl, Ld.y * sl, Ld.z * sl),
+              far ? __int_as_float(0x7f800000) : 1.0f, time);
       b.spath[si] = p;
       b.scontrib[si] = sc3.x;
       b.scontrib[b.cap + si] = sc3.y;
       b.scontrib[2 * (size_t)b.cap + si] = sc3.z;
       if (TRAIN) {
         const size_t c = b.cap;
-        b.snee[si] = rN.x; b.snee[c + si] = rN.y; b.snee[2 * c + si] = rN.z;
-        b.snee[3 * c + si] = rWi.x; b.snee[4 * c + si] = rWi.y; b.snee[5 * c + si] = rWi.z;
+        b.snee[si] = sc.N.x; b.snee[c + si] = sc.N.y; b.snee[2 * c + si] = sc.N.z;
+        b.snee[3 * c + si] = wi.x; b.snee[4 * c + si] = wi.y; b.snee[5 * c + si] = wi.z;
         b.snee[6 * c + si] = nee_w;
         b.snee[7 * c + si] = nee_pb;
       }
     }
-    const unsigned long long ni = warp_append(&b.qlen[d + 1], want_next);
-    if (want_next && ni < b.cap) {
-      put_ray(nq, b.cap, ni, no, nd, __int_as_float(0x7f800000), time);
+    const unsigned long long ni = warp_append(&b.qlen[d + 1], cont);
+    if (cont && ni < b.cap) {
+      put_ray(nq, b.cap, ni, so, wo, __int_as_float(0x7f800000), time);
       nqp[ni] = p;
     }
     if (TRAIN) {
@@ -720,7 +751,7 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : 3)) k_pt_
       if (want_rec && ri < b.rcap) {
         float* R = b.rec;
         const size_t c = b.rcap;
-        const float v[20] = {rP.x, rP.y, rP.z, rN.x, rN.y, rN.z, rWi.x, rWi.y, rWi.z, nd.x, nd.y, nd.z, 0.f, rQ,
+        const float v[20] = {sc.P.x, sc.P.y, sc.P.z, sc.N.x, sc.N.y, sc.N.z, wi.x, wi.y, wi.z, wo.x, wo.y, wo.z, 0.f, rQ,
                              b.bx[p], b.by[p], b.bz[p], 0.f, 0.f, 0.f};
         for (int k = 0; k < 20; ++k) R[(size_t)k * c + ri] = v[k];
         R[(size_t)kRPath * c + ri] = __uint_as_float(p);
@@ -990,6 +1021,8 @@ int launch_batch(vmr_ctx* ctx, const PtBatch& b, const DTop& top, DScratch* scr,
       }
     } else if (b.groups) {
       k_pt_shade<false, false, true><<<grid, kPtBlock, 0, st>>>(b, d);
+    } else if (b.cap >= kPtBigBatch) {
+      k_pt_shade<false, false, false, true><<<grid, kPtBlock, 0, st>>>(b, d);
     } else {
       k_pt_shade<false, false, false><<<grid, kPtBlock, 0, st>>>(b, d);
     }

@@ -473,10 +473,12 @@ __device__ __forceinline__ bool hit_attributes(const RMesh& m, int32_t prim, flo
   const float zs = fabsf(U * V0.z) + fabsf(V * V1.z) + fabsf(W * V2.z);
   const V3 e0 = sub(V1, V0), e1 = sub(V2, V0);
   const V3 Ng = normalize(v3(e0.y * e1.z - e0.z * e1.y, e0.z * e1.x - e0.x * e1.z, e0.x * e1.y - e0.y * e1.x));
-  V3 N = Ng;
+  sc.Ng = normalize(Ng);
+  sc.N = sc.Ng;  // without normals N is Ng
   if (m.nrm) {
     const float4 n0 = m.nrm[3 * (size_t)prim], n1 = m.nrm[3 * (size_t)prim + 1], n2 = m.nrm[3 * (size_t)prim + 2];
-    N = normalize(v3(U * n0.x + V * n1.x + W * n2.x, U * n0.y + V * n1.y + W * n2.y, U * n0.z + V * n1.z + W * n2.z));
+    sc.N = normalize(normalize(v3(U * n0.x + V * n1.x + W * n2.x, U * n0.y + V * n1.y + W * n2.y,
+                                  U * n0.z + V * n1.z + W * n2.z)));
   }
   const float g7 = (7.0f * 5.96046448e-08f) / (1 - 7.0f * 5.96046448e-08f);  // Gamma(7) (math/ferror.go:22-24)
   const float d = g7 * xs * fabsf(Ng.x) + g7 * ys * fabsf(Ng.y) + g7 * zs * fabsf(Ng.z);
@@ -486,8 +488,6 @@ __device__ __forceinline__ bool hit_attributes(const RMesh& m, int32_t prim, flo
   if (len2(axisu) < 0.1f || fabsf(dot(axisu, Ng)) > 0.3f) axisu = sub(v3(0, 0, 1), scale(dot(v3(0, 0, 1), Ng), Ng));
   const V3 dpdu = normalize(axisu);
   const V3 dpdv = cross(Ng, dpdu);
-  sc.N = normalize(N);
-  sc.Ng = normalize(Ng);
   sc.DdPdu = normalize(dpdu);
   sc.DdPdv = normalize(dpdv);
   return true;
@@ -621,7 +621,8 @@ __device__ __forceinline__ bool motion_attributes(const RMesh& m, int32_t elem, 
   const float d = g7 * xs * fabsf(Ng.x) + g7 * ys * fabsf(Ng.y) + g7 * zs * fabsf(Ng.z);
   sc.Poffset = scale(d, Ng);
   sc.P = v3(U * V0.x + V * V1.x + W * V2.x, U * V0.y + V * V1.y + W * V2.y, U * V0.z + V * V1.z + W * V2.z);
-  V3 N = Ng;
+  sc.Ng = normalize(Ng);
+  sc.N = sc.Ng;
   if (m.mnrm) {  // the element's corner normals of the two keys, lerped, then weighted by U, V, W
     V3 Nc[3];
     for (int j = 0; j < 3; ++j) {
@@ -629,11 +630,9 @@ __device__ __forceinline__ bool motion_attributes(const RMesh& m, int32_t elem, 
       const float4 a = m.mnrm[(size_t)key * m.mnrm_n + c], b = m.mnrm[(size_t)key2 * m.mnrm_n + c];
       Nc[j] = v3((1.0f - tm) * a.x + tm * b.x, (1.0f - tm) * a.y + tm * b.y, (1.0f - tm) * a.z + tm * b.z);
     }
-    N = normalize(v3(U * Nc[0].x + V * Nc[1].x + W * Nc[2].x, U * Nc[0].y + V * Nc[1].y + W * Nc[2].y,
-                     U * Nc[0].z + V * Nc[1].z + W * Nc[2].z));
+    sc.N = normalize(normalize(v3(U * Nc[0].x + V * Nc[1].x + W * Nc[2].x, U * Nc[0].y + V * Nc[1].y + W * Nc[2].y,
+                                  U * Nc[0].z + V * Nc[1].z + W * Nc[2].z)));
   }
-  sc.N = normalize(N);
-  sc.Ng = normalize(Ng);
   sc.DdPdu = normalize(e0);
   sc.DdPdv = normalize(e1);
   return true;
