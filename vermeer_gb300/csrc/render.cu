@@ -16,8 +16,8 @@
 //   trace         the any-hit kernel over the shadow queue
 //   k_accumulate  per pixel, the iterations in order: slots summed in the
 //                 reference's order, scaled, folded into the framebuffer
-// Transcendentals are evaluated in float64 and rounded to float32, as
-// math/sincos.go does; normalisation is a * (1/sqrt(a.a)) with IEEE sqrt and
+// Transcendentals are float64's values rounded to float32, as math/sincos.go
+// gives them (computed in float32 pairs, df32.cuh); normalisation is a * (1/sqrt(a.a)) with IEEE sqrt and
 // division (the reference's RSQRTSS estimate is machine-dependent).
 #include <cuda_runtime.h>
 
@@ -39,7 +39,7 @@ struct Cand {
   V3 Ld;
   float Ldist;
   float pdf_own;    // light samples: ls.Pdf; BSDF samples: unused
-  double pdf_bsdf;  // BSDF samples: bs.Pdf
+  float pdf_bsdf;   // BSDF samples: bs.Pdf
   float pdf_light;  // BSDF samples: bs.PdfLight
   bool ok;
 };
@@ -51,10 +51,12 @@ template <bool F32>
 __device__ Cand disk_sample(const RLight& L, const Ctx& sc, int n, int i) {
   Cand c{};
   const uint64_t idx = sc.I * (uint64_t)n + (uint64_t)i;
-  const double r0 = vdc(idx, sc.scr0), r1 = sobol(idx, sc.scr1);
-  const float u = L.radius * sqrtf((float)r0) * mcos<F32>(2 * kPi * (float)r1);
-  const float v = L.radius * sqrtf((float)r0) * msin<F32>(2 * kPi * (float)r1);
-  const double pdf = (double)(1.0f / (kPi * L.radius * L.radius));
+  const float r0 = frac52(vdc_bits(idx, sc.scr0)), r1 = frac52(sobol_bits(idx, sc.scr1));
+  float sn, cs;
+  msincos<F32>(2 * kPi * r1, sn, cs);
+  const float u = L.radius * sqrtf(r0) * cs;
+  const float v = L.radius * sqrtf(r0) * sn;
+  const float pdf = 1.0f / (kPi * L.radius * L.radius);
   const V3 LP = v3(L.P[0], L.P[1], L.P[2]), LT = v3(L.T[0], L.T[1], L.T[2]), LB = v3(L.B[0], L.B[1], L.B[2]),
            LN = v3(L.N[0], L.N[1], L.N[2]);
   const V3 P = add(add(LP, scale(u, LB)), scale(v, LT));
@@ -62,7 +64,7 @@ __device__ Cand disk_sample(const RLight& L, const Ctx& sc, int n, int i) {
   if (!(dot(V, sc.Ng) > 0.0f && dot(V, LN) < 0.0f)) return c;
   c.Ldist = length(V);
   c.Ld = normalize(V);
-  c.pdf_own = (float)pdf * (c.Ldist * c.Ldist) / fabsf(dot(c.Ld, LN));
+  c.pdf_own = pdf * (c.Ldist * c.Ldist) / fabsf(dot(c.Ld, LN));
   c.ok = true;
   return c;
 }
@@ -105,10 +107,12 @@ __device__ Cand sphere_sample(const RLight& L, const Ctx& sc, int n, int i) {
   const V3 v = normalize(cross(w, sc.Ng));
   const V3 u = cross(w, v);
   const uint64_t idx = sc.I * (uint64_t)n + (uint64_t)i;
-  const double r0 = vdc(idx, sc.scr0), r1 = sobol(idx, sc.scr1);
-  const float theta = macos<F32>(1 - (float)r0 + (float)r0 * sqrtf(1 - sqr(L.radius / l)));
-  const float phi = 2 * kPi * (float)r1;
-  const V3 a = v3(mcos<F32>(phi) * msin<F32>(theta), msin<F32>(phi) * msin<F32>(theta), mcos<F32>(theta));
+  const float r0 = frac52(vdc_bits(idx, sc.scr0)), r1 = frac52(sobol_bits(idx, sc.scr1));
+  const float theta = macos<F32>(1 - r0 + r0 * sqrtf(1 - sqr(L.radius / l)));
+  float sinT, cosT, sinP, cosP;
+  msincos<F32>(theta, sinT, cosT);
+  msincos<F32>(2 * kPi * r1, sinP, cosP);
+  const V3 a = v3(cosP * sinT, sinP * sinT, cosT);
   const V3 omega = expand(u, v, w, a);
   if (dot(omega, sc.Ng) < 0) return c;
   float t;
@@ -132,20 +136,25 @@ __device__ Cand light_sample(const RLight& L, const Ctx& sc, int n, int i) {
   const V3 N = normalize(cross(sub(p1, p0), sub(p2, p0)));
   const bool area_only = dot(sc.Ng, sub(p0, sc.P)) < 0 || dot(sc.Ng, sub(p1, sc.P)) < 0 || dot(sc.Ng, sub(p2, sc.P)) < 0;
   const uint64_t idx = sc.I * (uint64_t)n + (uint64_t)i;
-  const double r0 = vdc(idx, sc.scr0), r1 = sobol(idx, sc.scr1);
+  const uint64_t k0 = vdc_bits(idx, sc.scr0), k1 = sobol_bits(idx, sc.scr1);
   if (area_only) {
-    const double pdf = (double)(1 / tri_area(p0, p1, p2));
-    const float a = F32 ? (float)r1 * sqrtf(1.0f - (float)r0) : (float)(r1 * sqrt(1 - r0));
-    const float b = F32 ? 1.0f - sqrtf(1.0f - (float)r0) : (float)(1 - sqrt(1 - r0));
+    const float pdf = 1 / tri_area(p0, p1, p2);
+    float a, b;
+    if (F32) {
+      a = frac52(k1) * sqrtf(1.0f - frac52(k0));
+      b = 1.0f - sqrtf(1.0f - frac52(k0));
+    } else {
+      triangle_uv(k0, k1, a, b);
+    }
     const V3 P = add(add(p0, scale(a, sub(p1, p0))), scale(b, sub(p2, p0)));
     const V3 D = sub(P, sc.P);
     c.Ldist = length(D);
     c.Ld = normalize(D);
     if (dot(c.Ld, N) > 0 || dot(c.Ld, sc.Ng) < 0) return c;
-    c.pdf_own = (float)pdf * sqr(c.Ldist) / fabsf(dot(c.Ld, N));
+    c.pdf_own = pdf * sqr(c.Ldist) / fabsf(dot(c.Ld, N));
   } else {
-    double pdf;
-    const V3 x = sample_spherical<F32>(p0, p1, p2, sc.P, r0, r1, pdf);
+    float pdf;
+    const V3 x = sample_spherical<F32>(p0, p1, p2, sc.P, frac52(k0), frac52(k1), pdf);
     float t;
     ray_plane(sc.P, x, p0, N, t);
     const V3 P = add(sc.P, scale(t, x));
@@ -153,7 +162,7 @@ __device__ Cand light_sample(const RLight& L, const Ctx& sc, int n, int i) {
     c.Ldist = length(D);
     c.Ld = normalize(D);
     if (dot(c.Ld, N) > 0 || dot(c.Ld, sc.Ng) < 0) return c;
-    c.pdf_own = (float)pdf;
+    c.pdf_own = pdf;
   }
   c.ok = true;
   return c;
@@ -165,8 +174,7 @@ template <bool F32>
 __device__ Cand bsdf_candidate(const RLight& L, const Ctx& sc, const Bsdf& bsdf, int half, int i) {
   Cand c{};
   const uint64_t idx = sc.I * (uint64_t)half + (uint64_t)i;
-  const double r0 = vdc(idx, sc.scr0), r1 = sobol(idx, sc.scr1);
-  const V3 D = normalize(bsdf_sample<F32>(bsdf, r0, r1));
+  const V3 D = normalize(bsdf_sample<F32>(bsdf, vdc_bits(idx, sc.scr0), sobol_bits(idx, sc.scr1)));
   c.pdf_bsdf = bsdf_pdf<F32>(bsdf, D);
   if (c.pdf_bsdf <= 0) return c;
   if (L.kind == 2) {  // Sphere.ValidSample (sphere.go:126-176)
@@ -183,7 +191,7 @@ __device__ Cand bsdf_candidate(const RLight& L, const Ctx& sc, const Bsdf& bsdf,
     return c;
   }
   if (L.kind == 1) {
-    const double pdf = (double)(1.0f / (kPi * L.radius * L.radius));
+    const float pdf = 1.0f / (kPi * L.radius * L.radius);
     const V3 LP = v3(L.P[0], L.P[1], L.P[2]), LN = v3(L.N[0], L.N[1], L.N[2]);
     float t;
     if (!ray_plane(sc.P, D, LP, LN, t)) return c;  // rayDiskIntersect (disk.go:53-68)
@@ -194,7 +202,7 @@ __device__ Cand bsdf_candidate(const RLight& L, const Ctx& sc, const Bsdf& bsdf,
     if (dot(V, sc.Ng) <= 0.0f || dot(V, LN) >= 0.0f) return c;
     c.Ldist = length(V);
     c.Ld = normalize(V);
-    c.pdf_light = (float)pdf * (c.Ldist * c.Ldist) / fabsf(dot(c.Ld, LN));
+    c.pdf_light = pdf * (c.Ldist * c.Ldist) / fabsf(dot(c.Ld, LN));
     c.ok = true;
     return c;
   }
@@ -208,15 +216,15 @@ __device__ Cand bsdf_candidate(const RLight& L, const Ctx& sc, const Bsdf& bsdf,
   c.Ld = normalize(Dl);
   if (dot(c.Ld, N) > 0 || dot(c.Ld, sc.Ng) < 0) return c;
   if (area_only) {
-    const double pdf = (double)(1 / tri_area(p0, p1, p2));
-    c.pdf_light = (float)pdf * sqr(c.Ldist) / fabsf(dot(c.Ld, N));
+    const float pdf = 1 / tri_area(p0, p1, p2);
+    c.pdf_light = pdf * sqr(c.Ldist) / fabsf(dot(c.Ld, N));
   } else {
     const V3 pa = normalize(sub(p0, sc.P)), pb = normalize(sub(p1, sc.P)), pc = normalize(sub(p2, sc.P));
     const float a = macos<F32>(dot(pb, pc)), b = macos<F32>(dot(pc, pa)), cc = macos<F32>(dot(pa, pb));
     float al, be, ga;
     sides_to_angles<F32>(a, b, cc, al, be, ga);
     const float area = al + be + ga - kPi;
-    c.pdf_light = (float)(1 / (double)area);
+    c.pdf_light = 1 / area;
   }
   c.ok = true;
   return c;
@@ -362,10 +370,10 @@ __device__ float light_lobe(const RenderBatch& b, const Level& lv, const Ctx& sc
         if (mis) {
           float p_hat;
           if (pass == 0) {
-            p_hat = (float)nB * (float)bsdf_pdf<F32>(bsdf, c.Ld) / (float)total;
+            p_hat = (float)nB * bsdf_pdf<F32>(bsdf, c.Ld) / (float)total;
             p_hat += (float)nL * c.pdf_own / (float)total;
           } else {
-            p_hat = (float)nB * (float)c.pdf_bsdf / (float)total;
+            p_hat = (float)nB * c.pdf_bsdf / (float)total;
             p_hat += (float)nL * c.pdf_light / (float)total;
           }
           inv = 1.0f / p_hat;
@@ -394,8 +402,15 @@ __device__ float light_lobe(const RenderBatch& b, const Level& lv, const Ctx& sc
 // level: emission, the diffuse and glossy lobes' light samples, and the
 // mirror (Spec1Roughness 0) reflection queued for the next level with the
 // sample's I and scrambles (a child ShaderContext copies them).
+//
+// With the transcendentals in float64 this kernel was bound by that pipe (80%
+// busy, 2.72 ms for 1,048,576 samples of the small room at 164 registers); as
+// float32 pairs, and with Lambert's angles left out, 0.90 ms at 128 registers,
+// bound by instruction fetch.  8 resident blocks per SM (64 registers, a few
+// hundred bytes spilled) hide more of that than they cost: whole render 3.73
+// -> 3.63 ms (6 blocks 3.66, 5 3.70, 3 3.84); from float64 5.56 ms.
 template <bool F32, bool GROUPS>
-__global__ void __launch_bounds__(128) k_shade(RenderBatch b, uint32_t level) {
+__global__ void __launch_bounds__(128, GROUPS ? 1 : 8) k_shade(RenderBatch b, uint32_t level) {
   const Level& lv = b.lv[level];
   const uint64_t n = level == 0 ? (uint64_t)b.n : (*lv.count < lv.cap ? *lv.count : lv.cap);
   for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n; e += (uint64_t)gridDim.x * blockDim.x) {
@@ -489,15 +504,14 @@ __global__ void __launch_bounds__(128) k_shade(RenderBatch b, uint32_t level) {
       } else {
         // the mirror: one sample at idx = I (std.go:216-259)
         const Bsdf spec{2, sc.lambda, project(Ut, Vt, sc.N, wi), rough * rough, fr, Ut, Vt, sc.N};
-        const double r0 = vdc(sc.I, sc.scr0), r1 = sobol(sc.I, sc.scr1);
-        const V3 wo = bsdf_sample<F32>(spec, r0, r1);
-        const double pdf = bsdf_pdf<F32>(spec, wo);
+        const V3 wo = bsdf_sample<F32>(spec, vdc_bits(sc.I, sc.scr0), sobol_bits(sc.I, sc.scr1));
+        const float pdf = bsdf_pdf<F32>(spec, wo);
         float* w = lv.mw + e * 4;
         w[0] = w[1] = w[2] = 0.0f;
         w[3] = sw;
         if (dot(wo, sc.Ng) > 0.0f) {
           Spec rho = bsdf_eval<F32>(spec, wo);
-          const float inv = 1.0f / (float)pdf;
+          const float inv = 1.0f / pdf;
           for (int k = 0; k < 4; ++k) rho.c[k] *= inv;
           const RGB col = to_rgb(rho, sc.lambda);
           const RGB scol = (sh.flags & VMR_SH_SPEC1_COLOUR)

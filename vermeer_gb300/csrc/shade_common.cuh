@@ -6,8 +6,8 @@
 // each translation unit that includes it holds its own copy (including the
 // RasterXY constant tables, which each unit uploads).
 //
-// Transcendentals are evaluated in float64 and rounded to float32, as
-// math/sincos.go does; normalisation is a * (1/sqrt(a.a)) with IEEE sqrt and
+// Transcendentals are float64's values rounded to float32, as math/sincos.go
+// gives them (computed in float32 pairs, df32.cuh); normalisation is a * (1/sqrt(a.a)) with IEEE sqrt and
 // division (the reference's RSQRTSS estimate is machine-dependent).
 #pragma once
 #include <cuda_runtime.h>
@@ -17,6 +17,7 @@
 #include "animdecomp.h"
 #include "colour_tables.h"
 #include "ctx.h"
+#include "df32.cuh"
 #include "pixfilter.h"
 #include "vmr.h"
 
@@ -44,20 +45,26 @@ __device__ __forceinline__ float gmax(float x, float y) { return x > y ? x : y; 
 __device__ __forceinline__ float gmin(float x, float y) { return x < y ? x : y; }
 __device__ __forceinline__ float sqr(float v) { return v * v; }
 constexpr float kPi = 3.14159265358f;  // math.Pi (math/const.go:8) as float32
-__device__ __forceinline__ float gsin(float x) { return (float)sin((double)x); }
-__device__ __forceinline__ float gcos(float x) { return (float)cos((double)x); }
+__device__ __forceinline__ float gsin(float x) { return sin_rn(x); }
+__device__ __forceinline__ float gcos(float x) { return cos_rn(x); }
 __device__ __forceinline__ float gtan(float x) { return (float)tan((double)x); }
-__device__ __forceinline__ float gatan(float x) { return (float)atan((double)x); }
+__device__ __forceinline__ float gatan(float x) { return atan_rn(x); }
 __device__ __forceinline__ float gatan2(float y, float x) { return (float)atan2((double)y, (double)x); }
-__device__ __forceinline__ float gacos(float x) {
-  return (float)acos((double)(x > 1.0f ? 1.0f : (x < -1.0f ? -1.0f : x)));
-}
+__device__ __forceinline__ float gacos(float x) { return acos_rn(x > 1.0f ? 1.0f : (x < -1.0f ? -1.0f : x)); }
 // The same functions under the reference-mode precision switch: F32 false
 // is the float64 evaluation above (the reference's math/sincos.go, bit for
 // bit with the oracle); F32 true is CUDA's float32 functions (within 2 ulp),
 // the VMR_RENDER_F32 option, which keeps the shading off the FP64 pipe.
 template <bool F32> __device__ __forceinline__ float msin(float x) { return F32 ? sinf(x) : gsin(x); }
 template <bool F32> __device__ __forceinline__ float mcos(float x) { return F32 ? cosf(x) : gcos(x); }
+template <bool F32> __device__ __forceinline__ void msincos(float x, float& s, float& c) {
+  if (F32) {
+    s = sinf(x);
+    c = cosf(x);
+  } else {
+    sincos_rn(x, s, c);
+  }
+}
 template <bool F32> __device__ __forceinline__ float mtan(float x) { return F32 ? tanf(x) : gtan(x); }
 template <bool F32> __device__ __forceinline__ float matan(float x) { return F32 ? atanf(x) : gatan(x); }
 template <bool F32> __device__ __forceinline__ float matan2(float y, float x) { return F32 ? atan2f(y, x) : gatan2(y, x); }
@@ -237,22 +244,25 @@ __device__ __forceinline__ V3 reflect_z(V3 w) {
   return sub(scale(2.0f * d, v3(0, 0, 1)), w);
 }
 template <bool F32 = false>
-__device__ V3 bsdf_sample(const Bsdf& b, double r0, double r1) {
+__device__ V3 bsdf_sample(const Bsdf& b, uint64_t k0, uint64_t k1) {  // r0, r1 = k0, k1 / 2^52
   if (b.kind == 2) return expand(b.U, b.V, b.N, normalize(reflect_z(b.wi)));  // Specular.Sample
   if (b.kind == 0) {  // CosineHemisphere (math/sample/sample.go:18-27)
     if (F32) {
-      const float r = sqrtf(1.0f - (float)r0), th = 2.0f * kPi * (float)r1;
-      return expand(b.U, b.V, b.N, v3(r * cosf(th), r * sinf(th), sqrtf((float)r0)));
+      const float r0 = frac52(k0);
+      const float r = sqrtf(1.0f - r0), th = 2.0f * kPi * frac52(k1);
+      return expand(b.U, b.V, b.N, v3(r * cosf(th), r * sinf(th), sqrtf(r0)));
     }
-    const double r = sqrt(1 - r0), th = 2 * 3.14159265358979323846 * r1;
-    return expand(b.U, b.V, b.N, v3((float)(r * cos(th)), (float)(r * sin(th)), (float)sqrt(r0)));
+    V3 w;
+    cosine_hemisphere(k0, k1, w.x, w.y, w.z);
+    return expand(b.U, b.V, b.N, w);
   }
   const float alpha = sqr(b.rough);  // MicrofacetGGX.Sample
   float thetaM, phiM;
   if (F32) {
-    thetaM = atan2f(alpha * sqrtf((float)r0), sqrtf(1.0f - (float)r0));
-    phiM = 2.0f * kPi * (float)r1;
+    thetaM = atan2f(alpha * sqrtf(frac52(k0)), sqrtf(1.0f - frac52(k0)));
+    phiM = 2.0f * kPi * frac52(k1);
   } else {
+    const double r0 = frac52d(k0), r1 = frac52d(k1);
     thetaM = (float)atan2((double)alpha * sqrt(r0), sqrt(1 - r0));
     phiM = (float)(2.0 * 3.14159265358979323846 * r1);
   }
@@ -261,14 +271,14 @@ __device__ V3 bsdf_sample(const Bsdf& b, double r0, double r1) {
   return expand(b.U, b.V, b.N, normalize(wo));
 }
 template <bool F32 = false>
-__device__ double bsdf_pdf(const Bsdf& b, V3 wo_world) {
+__device__ float bsdf_pdf(const Bsdf& b, V3 wo_world) {  // float32 of the reference's float64
   const V3 wo = project(b.U, b.V, b.N, wo_world);
-  if (b.kind == 2) return dot(wo, reflect_z(b.wi)) < 0.9999f ? 0.0 : 1.0;  // Specular.PDF
-  if (b.kind == 0) return (double)gmax(0.0f, wo.z) / 3.14159265358979323846;
+  if (b.kind == 2) return dot(wo, reflect_z(b.wi)) < 0.9999f ? 0.0f : 1.0f;  // Specular.PDF
+  if (b.kind == 0) return over_pi(gmax(0.0f, wo.z));
   const float alpha = sqr(b.rough);
   const V3 m = scale(signf(b.wi.z), normalize(add(b.wi, wo)));
-  const double pdf = (double)(ggx_d(m, alpha) * m.z);
-  return isnan(pdf) ? 0.0 : pdf;
+  const float pdf = ggx_d(m, alpha) * m.z;
+  return isnan(pdf) ? 0.0f : pdf;
 }
 template <bool F32 = false>
 __device__ Spec bsdf_eval(const Bsdf& b, V3 wo_world) {
@@ -286,12 +296,15 @@ __device__ Spec bsdf_eval(const Bsdf& b, V3 wo_world) {
     const float sigma = b.rough;
     const float A = 1 - (0.5f * (sigma * sigma) / ((sigma * sigma) + 0.57f));
     const float B = 0.45f * (sigma * sigma) / ((sigma * sigma) + 0.09f);
-    const float phiI = matan2<F32>(b.wi.y, b.wi.x), phiO = matan2<F32>(wo.y, wo.x);
-    const float thetaI = macos<F32>(b.wi.z), thetaO = macos<F32>(wo.z);
-    const float alpha = gmax(thetaI, thetaO), beta = gmin(thetaI, thetaO);
-    const float C = msin<F32>(alpha) * mtan<F32>(beta);
-    const float gamma = mcos<F32>(phiO - phiI);
-    const float s = wo.z * (A + (B * gmax(0.0f, gamma) * C));
+    float s = wo.z;  // sigma 0 (Lambert): A = 1 and B = 0, whatever finite angles they would multiply
+    if (sigma != 0.0f || !isfinite(((b.wi.x + b.wi.y) + b.wi.z) + ((wo.x + wo.y) + wo.z))) {
+      const float phiI = matan2<F32>(b.wi.y, b.wi.x), phiO = matan2<F32>(wo.y, wo.x);
+      const float thetaI = macos<F32>(b.wi.z), thetaO = macos<F32>(wo.z);
+      const float alpha = gmax(thetaI, thetaO), beta = gmin(thetaI, thetaO);
+      const float C = msin<F32>(alpha) * mtan<F32>(beta);
+      const float gamma = mcos<F32>(phiO - phiI);
+      s = wo.z * (A + (B * gmax(0.0f, gamma) * C));
+    }
     Spec rho = from_rgb(RGB{{1, 1, 1}}, b.lambda);
 #pragma unroll
     for (int k = 0; k < 4; ++k) rho.c[k] *= s / kPi;
@@ -404,15 +417,16 @@ __device__ void sides_to_angles(float as, float bs, float cs, float& a, float& b
 }
 // sampleSphericalTriangle (triangle.go:474-535)
 template <bool F32 = false>
-__device__ V3 sample_spherical(V3 p0, V3 p1, V3 p2, V3 p, double r0, double r1, double& pdf) {
+__device__ V3 sample_spherical(V3 p0, V3 p1, V3 p2, V3 p, float r0, float r1, float& pdf) {
   const V3 pa = normalize(sub(p0, p)), pb = normalize(sub(p1, p)), pc = normalize(sub(p2, p));
   const float a = macos<F32>(dot(pb, pc)), b = macos<F32>(dot(pc, pa)), c = macos<F32>(dot(pa, pb));
   float alpha, beta, gamma;
   sides_to_angles<F32>(a, b, c, alpha, beta, gamma);
   const float area = alpha + beta + gamma - kPi;
-  const float areaHat = (float)r0 * area;
-  const float s = msin<F32>(areaHat - alpha), t = mcos<F32>(areaHat - alpha);
-  const float sinA = msin<F32>(alpha), cosA = mcos<F32>(alpha);
+  const float areaHat = r0 * area;
+  float s, t, sinA, cosA;
+  msincos<F32>(areaHat - alpha, s, t);
+  msincos<F32>(alpha, sinA, cosA);
   const float u = t - cosA;
   const float v = s + sinA * mcos<F32>(c);
   float q = ((v * t - u * s) * cosA - v) / ((v * s + u * t) * sinA);
@@ -421,10 +435,10 @@ __device__ V3 sample_spherical(V3 p0, V3 p1, V3 p2, V3 p, double r0, double r1, 
   const V3 v31 = normalize(v3(pc.x - w * pa.x, pc.y - w * pa.y, pc.z - w * pa.z));
   const float sq = sqrtf(1 - q * q);
   const V3 v4 = v3(q * pa.x + sq * v31.x, q * pa.y + sq * v31.y, q * pa.z + sq * v31.z);
-  const float z = 1 - (float)r1 * (1 - dot(v4, pb));
+  const float z = 1 - r1 * (1 - dot(v4, pb));
   w = dot(v4, pb);
   const V3 v42 = normalize(v3(v4.x - w * pb.x, v4.y - w * pb.y, v4.z - w * pb.z));
-  pdf = 1 / (double)area;
+  pdf = 1 / area;  // = float32 of the float64 quotient (twice 24 bits and two fit 53)
   return add(scale(z, pb), scale(sqrtf(1 - z * z), v42));
 }
 __device__ bool ray_plane(V3 Ro, V3 Rd, V3 P, V3 N, float& t) {
