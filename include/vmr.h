@@ -297,6 +297,13 @@ int vmr_trace_mesh(vmr_ctx* ctx, uint32_t geom, const vmr_rays* rays, size_t n, 
 /* Traversal of the two-level scene (Scene.Trace, scene.go:30-58). */
 int vmr_trace_scene(vmr_ctx* ctx, const vmr_rays* rays, size_t n, int flags,
                     const vmr_hits* hits, vmr_trace_stats* stats);
+/* The same two for n host rays stored one after the other, 8 floats each
+ * (px py pz dx dy dz tmax time); the device lays them out.  VMR_TRACE_DEVICE
+ * in flags: VMR_ERR_INVALID. */
+int vmr_trace_mesh_rows(vmr_ctx* ctx, uint32_t geom, const float* rows, size_t n, int flags,
+                        const vmr_hits* hits, vmr_trace_stats* stats);
+int vmr_trace_scene_rows(vmr_ctx* ctx, const float* rows, size_t n, int flags,
+                         const vmr_hits* hits, vmr_trace_stats* stats);
 
 /* Batched jobs (no reference counterpart: the reference renders one scene
  * per process).  Each job traces n rays against one mesh, static or motion;

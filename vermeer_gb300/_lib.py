@@ -183,6 +183,10 @@ SIGNATURES = {
                                       ctypes.POINTER(Hits), ctypes.POINTER(TraceStats)]),
     "vmr_trace_scene": (ctypes.c_int, [P, ctypes.POINTER(Rays), ctypes.c_size_t, ctypes.c_int,
                                        ctypes.POINTER(Hits), ctypes.POINTER(TraceStats)]),
+    "vmr_trace_mesh_rows": (ctypes.c_int, [P, U32, P, ctypes.c_size_t, ctypes.c_int,
+                                           ctypes.POINTER(Hits), ctypes.POINTER(TraceStats)]),
+    "vmr_trace_scene_rows": (ctypes.c_int, [P, P, ctypes.c_size_t, ctypes.c_int,
+                                            ctypes.POINTER(Hits), ctypes.POINTER(TraceStats)]),
     "vmr_set_shaders": (ctypes.c_int, [P, P, U32]),
     "vmr_mesh_set_shading": (ctypes.c_int, [P, U32, P, U32, P]),
     "vmr_mesh_set_motion_normals": (ctypes.c_int, [P, U32, P, U32, U32]),

@@ -303,8 +303,6 @@ class Context:
         if isinstance(rays, np.ndarray):
             rays = np.ascontiguousarray(rays, np.float32).reshape(-1, 8)
             n = rays.shape[0]
-            soa = np.ascontiguousarray(rays.T)
-            r = _lib.Rays(*[_p(soa[k]) for k in range(8)])
             out = {k: np.empty(n, np.int32 if k in ("prim", "geom") else np.float32) for k in outputs}
             h = _lib.Hits(*[_p(out.get(k)) for k in ("prim", "geom", "t", "u", "v", "w")])
         else:  # CUDA tensor [8, n], rows already in HBM
@@ -316,10 +314,12 @@ class Context:
                                   device=rays.device) for k in outputs}
             h = _lib.Hits(*[_p(out.get(k)) for k in ("prim", "geom", "t", "u", "v", "w")])
             flags |= TRACE_DEVICE
+        host = isinstance(rays, np.ndarray)
+        rest = (_p(rays) if host else ctypes.byref(r), n, flags, ctypes.byref(h), ctypes.byref(st))
         if geom is None:
-            rc = self.L.vmr_trace_scene(self.h, ctypes.byref(r), n, flags, ctypes.byref(h), ctypes.byref(st))
+            rc = (self.L.vmr_trace_scene_rows if host else self.L.vmr_trace_scene)(self.h, *rest)
         else:
-            rc = self.L.vmr_trace_mesh(self.h, geom, ctypes.byref(r), n, flags, ctypes.byref(h), ctypes.byref(st))
+            rc = (self.L.vmr_trace_mesh_rows if host else self.L.vmr_trace_mesh)(self.h, geom, *rest)
         self._check(rc)
         out["stats"] = dict(rays=st.rays, node_visits=st.node_visits, leaf_visits=st.leaf_visits,
                             tri_tests=st.tri_tests, kernel_ms=st.kernel_ms)

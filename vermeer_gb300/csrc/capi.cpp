@@ -399,27 +399,62 @@ int run_trace(vmr_ctx* ctx, const DMesh* mesh, const vmr_rays& r, size_t n, int 
   return st;
 }
 
+// The mesh that a mesh trace of geom walks.
+int trace_target(vmr_ctx* ctx, uint32_t geom, const DMesh** m) {
+  if (geom >= ctx->meshes.size()) return fail(ctx, VMR_ERR_INVALID, "bad geom id");
+  cudaSetDevice(ctx->device);
+  const MeshRec& rec = *ctx->meshes[geom];
+  if (rec.host.sphere || rec.host.group)
+    return fail(ctx, VMR_ERR_UNSUPPORTED, "sphere, instance and Proc geoms are traced through the scene (vmr_trace_scene)");
+  if (rec.host.n_tris == 0) return fail(ctx, VMR_ERR_INVALID, "empty mesh");
+  *m = &rec.dmesh;
+  return VMR_OK;
+}
+
 // Host-pointer trace: stage rays in, sort and trace, copy hits out, all
 // queued on ctx->stream; the status read after the downloads is the one
 // synchronisation.  (Splitting the call into chunks whose copies overlap the
 // neighbouring chunks' traversal measured slower on GB300: every persistent
 // launch ends with a tail in which SMs drain, and sorting smaller batches
 // groups rays less well, which cost more than the overlapped copies saved.)
-int trace_host(vmr_ctx* ctx, const DMesh* mesh, const vmr_rays* rays, size_t n, int flags, const vmr_hits* hits,
-               vmr_trace_stats* stats) {
+//
+// rows (rays is null then): rays of 8 floats each, which pass through a staging
+// buffer of kRowChunk rays and are laid out as arrays by the device.  (Transposed
+// by the host, a trace of 300,000 rays took 2.75 ms instead of 0.61.)
+constexpr size_t kRowChunk = 1u << 20;
+int trace_host(vmr_ctx* ctx, const DMesh* mesh, const vmr_rays* rays, const float* rows, size_t n, int flags,
+               const vmr_hits* hits, vmr_trace_stats* stats) {
   const size_t fb = n * sizeof(float);
-  const int n_in = rays->time ? 8 : 7;
-  const size_t bytes = fb * (size_t)n_in + fb * 6;
+  const int n_in = rows || rays->time ? 8 : 7;
+  const size_t arrays = fb * (size_t)n_in + fb * 6;
+  const size_t stage = rows ? (arrays + 15) / 16 * 16 : arrays;  // where the staged rows start
+  const size_t bytes = stage + (rows ? std::min(n, kRowChunk) * 32 : 0);
   VMR_CUDA(ctx, ctx->io.ensure(bytes == 0 ? 16 : bytes));
   char* base = ctx->io.as<char>();
-  const float* src[8] = {rays->px, rays->py, rays->pz, rays->dx, rays->dy, rays->dz, rays->tmax, rays->time};
   float* dst[8];
-  for (int k = 0; k < n_in; ++k) {
-    dst[k] = reinterpret_cast<float*>(base + fb * k);
-    if (!src[k]) return fail(ctx, VMR_ERR_INVALID, "null ray array");
+  for (int k = 0; k < n_in; ++k) dst[k] = reinterpret_cast<float*>(base + fb * k);
+  if (rows) {
+    float* staged = reinterpret_cast<float*>(base + stage);
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 0; i < n && e == cudaSuccess; i += kRowChunk) {
+      const size_t m = std::min(n - i, kRowChunk);
+      e = cudaMemcpyAsync(staged, rows + 8 * i, m * 32, cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess)
+        e = (cudaError_t)vmr::launch_ray_columns(
+            staged, m, vmr::RaySoA{dst[0] + i, dst[1] + i, dst[2] + i, dst[3] + i, dst[4] + i, dst[5] + i, dst[6] + i, dst[7] + i},
+            ctx->stream);
+    }
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(ctx->stream);
+      return cuda_fail(ctx, e, "ray upload");
+    }
+  } else {
+    const float* src[8] = {rays->px, rays->py, rays->pz, rays->dx, rays->dy, rays->dz, rays->tmax, rays->time};
+    for (int k = 0; k < n_in; ++k)
+      if (!src[k]) return fail(ctx, VMR_ERR_INVALID, "null ray array");
+    for (int k = 0; k < n_in; ++k)
+      if (n) VMR_CUDA(ctx, cudaMemcpyAsync(dst[k], src[k], fb, cudaMemcpyHostToDevice, ctx->stream));
   }
-  for (int k = 0; k < n_in; ++k)
-    if (n) VMR_CUDA(ctx, cudaMemcpyAsync(dst[k], src[k], fb, cudaMemcpyHostToDevice, ctx->stream));
   char* hb = base + fb * n_in;
   void* outs[6] = {hits->prim, hits->geom, hits->t, hits->u, hits->v, hits->w};
   char* douts[6];
@@ -987,14 +1022,10 @@ int vmr_trace_mesh(vmr_ctx* ctx, uint32_t geom, const vmr_rays* rays, size_t n, 
                    vmr_trace_stats* stats) {
   if (ctx && ctx->device < 0) return fail(ctx, VMR_ERR_UNSUPPORTED, "host-only context cannot trace");
   if (!ctx || !rays || !hits) return VMR_ERR_INVALID;
-  if (geom >= ctx->meshes.size()) return fail(ctx, VMR_ERR_INVALID, "bad geom id");
-  cudaSetDevice(ctx->device);
-  const DMesh* m = &ctx->meshes[geom]->dmesh;
-  if (ctx->meshes[geom]->host.sphere || ctx->meshes[geom]->host.group)
-    return fail(ctx, VMR_ERR_UNSUPPORTED, "sphere, instance and Proc geoms are traced through the scene (vmr_trace_scene)");
-  if (ctx->meshes[geom]->host.n_tris == 0) return fail(ctx, VMR_ERR_INVALID, "empty mesh");
+  const DMesh* m = nullptr;
+  if (int rc = trace_target(ctx, geom, &m)) return rc;
   if (flags & VMR_TRACE_DEVICE) return run_trace(ctx, m, *rays, n, flags, *hits, stats);
-  return trace_host(ctx, m, rays, n, flags, hits, stats);
+  return trace_host(ctx, m, rays, nullptr, n, flags, hits, stats);
 }
 
 int vmr_trace_scene(vmr_ctx* ctx, const vmr_rays* rays, size_t n, int flags, const vmr_hits* hits,
@@ -1004,9 +1035,28 @@ int vmr_trace_scene(vmr_ctx* ctx, const vmr_rays* rays, size_t n, int flags, con
   if (!ctx->top.valid) return fail(ctx, VMR_ERR_INVALID, "no scene: call vmr_scene_build first");
   cudaSetDevice(ctx->device);
   if (flags & VMR_TRACE_DEVICE) return run_trace(ctx, nullptr, *rays, n, flags, *hits, stats);
-  return trace_host(ctx, nullptr, rays, n, flags, hits, stats);
+  return trace_host(ctx, nullptr, rays, nullptr, n, flags, hits, stats);
 }
 
+int vmr_trace_mesh_rows(vmr_ctx* ctx, uint32_t geom, const float* rows, size_t n, int flags, const vmr_hits* hits,
+                        vmr_trace_stats* stats) {
+  if (ctx && ctx->device < 0) return fail(ctx, VMR_ERR_UNSUPPORTED, "host-only context cannot trace");
+  if (!ctx || !rows || !hits) return VMR_ERR_INVALID;
+  if (flags & VMR_TRACE_DEVICE) return fail(ctx, VMR_ERR_INVALID, "vmr_trace_mesh_rows takes host rays");
+  const DMesh* m = nullptr;
+  if (int rc = trace_target(ctx, geom, &m)) return rc;
+  return trace_host(ctx, m, nullptr, rows, n, flags, hits, stats);
+}
+
+int vmr_trace_scene_rows(vmr_ctx* ctx, const float* rows, size_t n, int flags, const vmr_hits* hits,
+                         vmr_trace_stats* stats) {
+  if (ctx && ctx->device < 0) return fail(ctx, VMR_ERR_UNSUPPORTED, "host-only context cannot trace");
+  if (!ctx || !rows || !hits) return VMR_ERR_INVALID;
+  if (flags & VMR_TRACE_DEVICE) return fail(ctx, VMR_ERR_INVALID, "vmr_trace_scene_rows takes host rays");
+  if (!ctx->top.valid) return fail(ctx, VMR_ERR_INVALID, "no scene: call vmr_scene_build first");
+  cudaSetDevice(ctx->device);
+  return trace_host(ctx, nullptr, nullptr, rows, n, flags, hits, stats);
+}
 
 int vmr_clear_tuning(vmr_ctx* ctx, uint32_t geom) {
   if (!ctx || geom >= ctx->meshes.size()) return VMR_ERR_INVALID;

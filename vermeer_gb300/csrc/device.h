@@ -213,6 +213,8 @@ int launch_trace_mesh(const DMesh& mesh, const TraceLaunch& l);
 int launch_ray_sort(const RaySoA& rays, uint64_t n, const float bounds[6], int bits, uint32_t* keys, uint32_t* hist,
                     uint32_t* order, const RaySoA& sorted_out, void* stream,
                     const unsigned long long* n_dev = nullptr);
+// n rays of 8 floats (16-byte aligned device memory) -> out's eight arrays.
+int launch_ray_columns(const float* rows, uint64_t n, const RaySoA& out, void* stream);
 int launch_trace_scene(const DTop& top, const TraceLaunch& l);
 // out[8][n]: the octant copies of n nodes (traverse.cu).
 int launch_octant_nodes(const GNode* nodes, uint32_t n, ONode* out, void* stream);

@@ -460,11 +460,12 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_guide_infer(GuideRows in, 
     const bool valid = row < n;
     float q[3] = {0.f, 0.f, 0.f}, nn[3] = {0.f, 0.f, 0.f}, wo[3] = {0.f, 0.f, 0.f};
     if (valid) {
-      q[0] = (in.px[row] - in.lo[0]) * in.inv_ext[0];
-      q[1] = (in.py[row] - in.lo[1]) * in.inv_ext[1];
-      q[2] = (in.pz[row] - in.lo[2]) * in.inv_ext[2];
-      nn[0] = in.nx[row]; nn[1] = in.ny[row]; nn[2] = in.nz[row];
-      wo[0] = in.wx[row]; wo[1] = in.wy[row]; wo[2] = in.wz[row];
+      const uint64_t e = row * in.vstride;
+      q[0] = (in.px[e] - in.lo[0]) * in.inv_ext[0];
+      q[1] = (in.py[e] - in.lo[1]) * in.inv_ext[1];
+      q[2] = (in.pz[e] - in.lo[2]) * in.inv_ext[2];
+      nn[0] = in.nx[e]; nn[1] = in.ny[e]; nn[2] = in.nz[e];
+      wo[0] = in.wx[e]; wo[1] = in.wy[e]; wo[2] = in.wz[e];
     }
 #pragma unroll 1
     for (uint32_t ax = 0; ax < 3; ++ax) put_axis_features(a, r, ax, ax == 0 ? q[0] : (ax == 1 ? q[1] : q[2]), valid);
@@ -597,16 +598,16 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_guide_train(GuideTrain tr,
       float f[80];
       if (valid) {
         const GuideRows& in = tr.rows;
-        const uint64_t e = row * in.rstride;
+        const uint64_t e = row * in.vstride, es = row * tr.sstride;
         const float p[3] = {in.px[e], in.py[e], in.pz[e]};
         const float nn[3] = {in.nx[e], in.ny[e], in.nz[e]};
         const float wo[3] = {in.wx[e], in.wy[e], in.wz[e]};
         features(p, nn, wo, in.lo, in.inv_ext, f);
-        weight = tr.weight[e];
+        weight = tr.weight[es];
         om[0] = tr.ox[e];
         om[1] = tr.oy[e];
         om[2] = tr.oz[e];
-        if (tr.pb) pb = tr.pb[e];
+        if (tr.pb) pb = tr.pb[es];
       } else {
         for (int k = 0; k < 80; ++k) f[k] = 0.f;
       }
@@ -963,6 +964,11 @@ int gfail(vmr_ctx* ctx, int code, const std::string& msg) {
   ctx->err = msg;
   return code;
 }
+// Waits, on every way out of a call, for the copies that still read its caller's arrays.
+struct Drain {
+  cudaStream_t st;
+  ~Drain() { cudaStreamSynchronize(st); }
+};
 #define GCUDA(x)                                                               \
   do {                                                                         \
     cudaError_t e_ = (x);                                                      \
@@ -1018,49 +1024,44 @@ int guide_check(vmr_ctx* ctx) {
   return VMR_OK;
 }
 
-// Host n x 3 arrays -> device SoA rows in the context's staging buffer
-// (omega, weight and pb optional), followed by extra_out floats of room.
+// Host n x 3 arrays (omega, weight and pb optional) -> the context's staging
+// buffer, as they are: the kernels read the rows in place.  (Transposed to
+// columns by the host first, through a fresh buffer, a vmr_guide_gradient of 65,536
+// records took 744 us instead of 236.)  extra_out floats of room follow.  The copies
+// may still read the arrays when this returns: the caller holds a Drain.
 int stage_rows(vmr_ctx* ctx, const float* pos, const float* nrm, const float* wo, const float* omega,
                const float* weight, const float* pb, size_t n, const float lo[3], const float hi[3], GuideTrain& tr,
                size_t extra_out) {
   auto& G = ctx->guide;
   const size_t cols = 9 + (omega ? 3 : 0) + (weight ? 1 : 0) + (pb ? 1 : 0);
   GCUDA(G.io.ensure((cols * n + extra_out) * sizeof(float) + 256));
-  std::vector<float> h(cols * n);
-  for (size_t i = 0; i < n; ++i)
-    for (int c = 0; c < 3; ++c) {
-      h[c * n + i] = pos[3 * i + c];
-      h[(3 + c) * n + i] = nrm[3 * i + c];
-      h[(6 + c) * n + i] = wo[3 * i + c];
-      if (omega) h[(9 + c) * n + i] = omega[3 * i + c];
-    }
-  size_t col = omega ? 12 : 9;
-  const size_t wcol = col;
-  if (weight) {
-    for (size_t i = 0; i < n; ++i) h[col * n + i] = weight[i];
-    ++col;
-  }
-  const size_t pcol = col;
-  if (pb)
-    for (size_t i = 0; i < n; ++i) h[col * n + i] = pb[i];
   float* d = G.io.as<float>();
-  GCUDA(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-  GCUDA(cudaStreamSynchronize(ctx->stream));  // h goes out of scope
+  cudaError_t e = cudaSuccess;
+  auto put = [&](const float* src, size_t width) -> const float* {
+    if (!src) return nullptr;
+    const float* at = d;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, src, width * n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
+    d += width * n;
+    return at;
+  };
+  const float *p = put(pos, 3), *nn = put(nrm, 3), *w = put(wo, 3), *o = put(omega, 3);
+  tr.weight = put(weight, 1);
+  tr.pb = put(pb, 1);
+  if (e != cudaSuccess) return gfail(ctx, VMR_ERR_CUDA, cudaGetErrorString(e));
   GuideRows& r = tr.rows;
-  r.px = d; r.py = d + n; r.pz = d + 2 * n;
-  r.nx = d + 3 * n; r.ny = d + 4 * n; r.nz = d + 5 * n;
-  r.wx = d + 6 * n; r.wy = d + 7 * n; r.wz = d + 8 * n;
+  r.px = p; r.py = p + 1; r.pz = p + 2;
+  r.nx = nn; r.ny = nn + 1; r.nz = nn + 2;
+  r.wx = w; r.wy = w + 1; r.wz = w + 2;
+  r.vstride = 3;
   r.n = n;
   r.n_dev = nullptr;
   for (int c = 0; c < 3; ++c) {
     r.lo[c] = lo[c];
     r.inv_ext[c] = 1.0f / (hi[c] - lo[c]);
   }
-  if (omega) {
-    tr.ox = d + 9 * n; tr.oy = d + 10 * n; tr.oz = d + 11 * n;
+  if (o) {
+    tr.ox = o; tr.oy = o + 1; tr.oz = o + 2;
   }
-  if (weight) tr.weight = d + wcol * n;
-  tr.pb = pb ? d + pcol * n : nullptr;
   tr.stride = (uint32_t)n;
   return VMR_OK;
 }
@@ -1197,6 +1198,7 @@ int vmr_guide_forward(vmr_ctx* ctx, const float* pos, const float* nrm, const fl
   // the outputs follow the 9 input columns: 9n floats, a multiple of 16 bytes
   // when the row count is (padded below)
   const size_t n4 = (n + 3) / 4 * 4;
+  const Drain drain{ctx->stream};
   rc = stage_rows(ctx, pos, nrm, wo, nullptr, nullptr, nullptr, n, lo, hi, tr, 9 * (n4 - n) + n * kGuideOutStride);
   if (rc) return rc;
   float* dout = ctx->guide.io.as<float>() + 9 * n4;
@@ -1223,6 +1225,7 @@ int vmr_guide_gradient(vmr_ctx* ctx, const float* pos, const float* nrm, const f
   GuideTrain tr{};
   if (bsdf_pdf && !(alpha_max > 0.0f && alpha_max < 1.0f))
     return gfail(ctx, VMR_ERR_INVALID, "alpha_max must be in (0, 1)");
+  const Drain drain{ctx->stream};
   rc = stage_rows(ctx, pos, nrm, wo, omega, weight, bsdf_pdf, n, lo, hi, tr, 0);
   tr.amax = alpha_max;
   if (rc) return rc;
@@ -1250,6 +1253,7 @@ int vmr_guide_train_step(vmr_ctx* ctx, const float* pos, const float* nrm, const
   GuideTrain tr{};
   if (bsdf_pdf && !(alpha_max > 0.0f && alpha_max < 1.0f))
     return gfail(ctx, VMR_ERR_INVALID, "alpha_max must be in (0, 1)");
+  const Drain drain{ctx->stream};
   rc = stage_rows(ctx, pos, nrm, wo, omega, weight, bsdf_pdf, n, lo, hi, tr, 0);
   tr.amax = alpha_max;
   if (rc) return rc;

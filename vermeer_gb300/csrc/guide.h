@@ -14,27 +14,29 @@ constexpr int kGuideOutStride = 44;  // floats per row of an inference output
 constexpr uint32_t kSaveRows = 640;   // values saved per training record (chunk-blocked)
 
 // Path vertices (SoA, device pointers): hit point, shading normal, direction
-// toward the previous vertex; n rows, or *n_dev rows when n_dev is set.  The
-// training kernel reads row r at element r * rstride of every array
-// (inference reads rows contiguously).
+// toward the previous vertex; n rows, or *n_dev rows when n_dev is set.  Row r
+// of a vector component is element r * vstride of its array (3: a host
+// caller's n x 3 rows, copied as they are).
 struct GuideRows {
   const float *px, *py, *pz, *nx, *ny, *nz, *wx, *wy, *wz;
   uint64_t n;
   const unsigned long long* n_dev;
   float lo[3], inv_ext[3];  // scene bounds: q = (p - lo) * inv_ext
-  uint32_t rstride = 1;
+  uint32_t vstride = 1;
 };
 
 // Training records: the rows plus the sampled direction and its weight
 // (incident radiance over the density it was sampled with), and optionally
 // the BSDF's density of that direction: with it the loss is that of the
 // vertex's full sampling density alpha p_guide + (1 - alpha) p_bsdf, alpha =
-// amax * sigmoid(selection logit), which also trains the selection.
+// amax * sigmoid(selection logit), which also trains the selection.  Row r of
+// weight and pb is element r * sstride.
 struct GuideTrain {
   GuideRows rows;
   const float *ox, *oy, *oz, *weight;
   const float* pb;  // nullptr: the guide's own density
   float amax;
+  uint32_t sstride = 1;
   uint32_t stride;  // records the save buffer holds (a multiple of 128)
 };
 

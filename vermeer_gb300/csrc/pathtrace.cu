@@ -1514,7 +1514,7 @@ static int render_path_impl(vmr_ctx* ctx, const vmr_path_params* p, float* fb, v
         tr.rows.wx = R + kRWo * c + off; tr.rows.wy = R + (kRWo + 1) * c + off; tr.rows.wz = R + (kRWo + 2) * c + off;
         tr.rows.n = tbatch;
         tr.rows.n_dev = ncount;
-        tr.rows.rstride = tsteps;
+        tr.rows.vstride = tr.sstride = tsteps;
         tr.ox = R + kROm * c + off; tr.oy = R + (kROm + 1) * c + off; tr.oz = R + (kROm + 2) * c + off;
         tr.weight = R + kRW * c + off;
         tr.pb = learn_sel ? R + kRPb * c + off : nullptr;

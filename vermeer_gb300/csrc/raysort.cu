@@ -175,7 +175,27 @@ __global__ void k_ray_scatter(RaySoA rays, uint64_t n, const unsigned long long*
   }
 }
 
+// Host callers' rays, 32 bytes each, to arrays.  Bound by memory: a warp reads
+// 1 KB of rays and writes a whole line of each array.
+__global__ void k_ray_columns(const float4* __restrict__ rows, uint64_t n, float* px, float* py, float* pz, float* dx,
+                              float* dy, float* dz, float* tmax, float* time) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const float4 a = rows[2 * i], b = rows[2 * i + 1];
+    px[i] = a.x; py[i] = a.y; pz[i] = a.z; dx[i] = a.w;
+    dy[i] = b.x; dz[i] = b.y; tmax[i] = b.z; time[i] = b.w;
+  }
+}
+
 }  // namespace
+
+int launch_ray_columns(const float* rows, uint64_t n, const RaySoA& out, void* stream) {
+  const uint64_t want = (n + 255) / 256, cap = (uint64_t)device_sm_count() * 8;
+  auto w = [](const float* p) { return const_cast<float*>(p); };
+  k_ray_columns<<<(int)(want < cap ? want : cap), 256, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const float4*>(rows), n, w(out.px), w(out.py), w(out.pz), w(out.dx), w(out.dy), w(out.dz),
+      w(out.tmax), w(out.time));
+  return (int)cudaGetLastError();
+}
 
 int launch_ray_sort(const RaySoA& rays, uint64_t n, const float bounds[6], int bits, uint32_t* keys, uint32_t* hist,
                     uint32_t* order, const RaySoA& sorted_out, void* stream, const unsigned long long* n_dev) {
