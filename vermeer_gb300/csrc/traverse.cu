@@ -31,6 +31,8 @@
 // k_jobs_scatter (vmr_trace_jobs).
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "device.h"
 
 namespace vmr {
@@ -1125,24 +1127,37 @@ __global__ void k_octant_nodes(const GNode* __restrict__ nodes, uint32_t n, ONod
 
 // A traversal stack whose first SS entries per thread live in shared memory
 // (entry-major, so the 32 lanes of a warp always touch 32 different banks)
-// and the rest in local memory; SS = 0 keeps the whole stack local.
-template <int SS>
+// and the rest in local memory; SS = 0 keeps the whole stack local.  TS: the
+// entries carry T.
+template <int SS, bool TS>
 struct SplitStack {
   int* sn;     // shared node ids: entry k of this thread at sn[k * stride]
   float* st;   // shared T values
   int stride;  // threads per block
-  int2 loc[kStackCapacity - SS];
+  using Entry = typename std::conditional<TS, int2, int>::type;
+  Entry loc[kStackCapacity - SS];
   __device__ __forceinline__ void set(int i, int node, float T) {
     if (SS > 0 && i < SS) {
       sn[i * stride] = node;
-      st[i * stride] = T;
+      if (TS) st[i * stride] = T;
     } else {
-      loc[i - SS] = make_int2(node, __float_as_int(T));
+      if constexpr (TS) loc[i - SS] = make_int2(node, __float_as_int(T));
+      else loc[i - SS] = node;
     }
   }
-  __device__ __forceinline__ int2 get(int i) const {
-    if (SS > 0 && i < SS) return make_int2(sn[i * stride], __float_as_int(st[i * stride]));
-    return loc[i - SS];
+  // The node; T too where the entries carry it.
+  __device__ __forceinline__ int get(int i, float& T) const {
+    if (SS > 0 && i < SS) {
+      if (TS) T = st[i * stride];
+      return sn[i * stride];
+    }
+    if constexpr (TS) {
+      const int2 e = loc[i - SS];
+      T = __int_as_float(e.y);
+      return e.x;
+    } else {
+      return loc[i - SS];
+    }
   }
 };
 
@@ -1517,7 +1532,10 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
   extern __shared__ int stack_smem[];
   // a leaf phase's leaves of each warp by rank: lane, first triangle - first position
   __shared__ int2 leaf_map[COOP ? (MINB > 0 ? 128 : 256) : 1];
-  SplitStack<SS> stk;
+  // A shadow ray's Tclosest holds until its traversal ends, and what was pushed was
+  // not behind it: nothing is culled at a pop, and its 4-byte entries halve the
+  // stack's L1 traffic (600,011 rays 477 -> 467 us).
+  SplitStack<SS, !ANY> stk;
   if (SS > 0) {
     stk.stride = blockDim.x;
     stk.sn = stack_smem + threadIdx.x;
@@ -1613,9 +1631,9 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
           node = -1;
           return;
         }
-        const int2 e = stk.get(--sp);
-        node = e.x;
-        if (!(r.tclosest < __int_as_float(e.y))) return;
+        float T = 0.f;
+        node = stk.get(--sp, T);
+        if (ANY || !(r.tclosest < T)) return;
       }
     };
     if (alive) {
