@@ -247,5 +247,30 @@ __device__ __forceinline__ void triangle_uv(uint64_t k0, uint64_t k1, float& a, 
   if (!(oka && okb)) triangle_uv64(k0, k1, a, b);
 }
 
+// The camera sample's float64 expressions (core/render.go), rounded.
+// (float)(-1 + 2 r / w), r = k / 2^40: 2 k - 2^40 w is exact, and float64's
+// errors are below 2^-51 of 2 r / w + 1.
+__device__ __noinline__ float raster_ndc64(uint64_t k, uint32_t w) {
+  return (float)(-1.0 + 2.0 * ((double)k / 1099511627776.0 / (double)w));
+}
+__device__ __forceinline__ float raster_ndc(uint64_t k, uint32_t w) {
+  if (w < (1u << 22)) {
+    const DF n = df_int((int64_t)(2 * k) - ((int64_t)w << 40));
+    const float fw = (float)w, rw = 1.0f / fw, q = n.h * rw;
+    const DF v = df_fast(q * 0x1p-40f, (__fmaf_rn(-q, fw, n.h) + n.l) * rw * 0x1p-40f);
+    float f;
+    if (df_round(v, __fmaf_rn(kDfErr, fabsf(v.h), 0x1p-49f), f)) return f;
+  }
+  return raster_ndc64(k, w);
+}
+// (float)(270 v + 450), v = k / 2^52: the exact sum over 2^52; float64's two
+// roundings move it by less than 2^-52 * 512.
+__device__ __noinline__ float wavelength64(uint64_t k) { return (float)((720.0 - 450.0) * frac52d(k) + 450.0); }
+__device__ __forceinline__ float wavelength52(uint64_t k) {
+  const int64_t n = 270 * (int64_t)k + (450ll << 52);
+  const float a = __ll2float_rn(n - 512), b = __ll2float_rn(n + 512);
+  return a == b ? a * 0x1p-52f : wavelength64(k);
+}
+
 }  // namespace
 }  // namespace vmr

@@ -396,8 +396,9 @@ __global__ void __launch_bounds__(kPtBlock) k_pt_generate(PtBatch b) {
   const uint64_t n = b.it->n < b.cap ? b.it->n : b.cap;
   if (blockIdx.x == 0 && threadIdx.x == 0) b.qlen[0] = n;
   for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < n; s += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t pix = (uint32_t)(s % b.npix);
-    const uint32_t j = b.it->iter0 + (uint32_t)(s / b.npix) + 1;
+    const uint32_t it = (uint32_t)s / b.npix;  // s < cap, 32 bits
+    uint32_t pix = (uint32_t)s - it * b.npix;
+    const uint32_t j = b.it->iter0 + it + 1;
     V3 P, D;
     float time, lambda;
     if (b.n_jobs) {  // the job holding arena pixel pix (jobs sorted by pix0)

@@ -292,8 +292,9 @@ template <bool CKEYS>
 __global__ void k_generate(RenderBatch b) {
   const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (s >= b.n) return;
-  const uint32_t pix = b.pix0 + (uint32_t)(s % b.npix);    // the image pixel
-  const uint32_t j = b.iter0 + (uint32_t)(s / b.npix) + 1;  // render(iter+1)
+  const uint32_t it = s >> 32 ? (uint32_t)(s / b.npix) : (uint32_t)s / b.npix;
+  const uint32_t pix = b.pix0 + (uint32_t)(s - (uint64_t)it * b.npix);  // the image pixel
+  const uint32_t j = b.iter0 + it + 1;                                  // render(iter+1)
   V3 P, D;
   float time, lambda;
   camera_primary<CKEYS>(b.cam, b.cam_keys, b.cam_nkeys, b.width, b.height, j, pix, b.seed, b.filt, P, D, time,
