@@ -45,3 +45,27 @@ def test_queue_sort_with_an_odd_number_of_paths(ctx):
     a, _ = ctx.render_path(257, 257, 0, 1, 5, max_depth=3)
     b, _ = ctx.render_path(257, 257, 0, 1, 5, max_depth=3, sort_queues=True)
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [65536, 70001])
+def test_sorted_scene_records_equal_unsorted(ctx, n):
+    """Several meshes and a sphere, which reads the ray again: record copies
+    against the rays in input order."""
+    from vermeer_gb300 import scenes
+    geoms = [ctx.mesh_build(*scenes.triangle_soup(800, 45 + k, edge=0.08)) for k in range(2)]
+    geoms.append(ctx.sphere_add((0.5, 0.5, 0.5), 0.2))
+    ctx.scene_build(geoms)
+    rays = scenes.incoherent_rays(n, 48)
+    rays[1::3, 6] = 0.4  # some with a finite reach
+    try:
+        for shadow in (False, True):
+            got = []
+            for kernel in (45 & ~8, 45, 45 & ~32):
+                ctx.set_tuning(kernel=kernel)
+                got.append(ctx.trace_scene(rays, shadow=shadow))
+            assert (got[0]["geom"] == geoms[2]).any() and (got[0]["geom"] == geoms[0]).any()
+            for g in got[1:]:
+                for k in ("prim", "geom", "t", "u", "v", "w"):
+                    assert np.array_equal(got[0][k].view(np.uint32), g[k].view(np.uint32)), (k, shadow)
+    finally:
+        ctx.set_tuning()

@@ -364,11 +364,13 @@ int launch_trace_chunk(vmr_ctx* ctx, const DMesh* mesh, const vmr_rays& r, size_
     // which is no context mesh, covers exactly the scene's geoms)
     const float* mb = mesh ? ctx->mesh_bounds_of(mesh) : ctx->top.bounds6;
     if (!mb) mb = ctx->top.bounds6;
-    // A static mesh in the while-while kernel reads the copy as 32-byte
-    // records (two 16-byte loads a ray, its input index inside), written
-    // over the order and array regions (4 + 28 bytes a ray); a static mesh reads
-    // no ray times.
-    const bool recs = mesh && mesh->keys <= 1 && (tn.kernel & vmr::kKernelWhileWhile);
+    // Static meshes and scenes in the while-while kernels read the copy as
+    // 32-byte records (two 16-byte loads a ray, its input index inside),
+    // written over the order and array regions (4 + 28 bytes a ray); they
+    // read no ray times.  (scene_sort: a static scene, no visit counters;
+    // 1,000,003 rays on the sphere grid 455 -> 421 us against arrays, whose
+    // eight scattered 4-byte stores a ray touch a sector each.)
+    const bool recs = (!mesh || mesh->keys <= 1) && (tn.kernel & vmr::kKernelWhileWhile);
     if (recs) sorted = vmr::RaySoA{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, order};
     int se = vmr::launch_ray_sort(l.rays, n, mb, tn.sort_bits ? tn.sort_bits : vmr::default_sort_bits(n), keys, hist, order, sorted,
                                   ctx->stream);

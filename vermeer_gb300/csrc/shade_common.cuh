@@ -107,7 +107,7 @@ __constant__ uint64_t c_raster_inv[52];
 // raster coordinates are kx, ky / 2^40.
 //
 // The camera kernels were bound by the float64 pipe (83% busy, 490 us for
-// 3,686,400 samples) and by the bit loops here and in sobol_bits (2,600
+// 8,294,400 samples) and by the bit loops here and in sobol_bits (1,200
 // instructions a sample).  The sample's coordinates stay integers, its float32
 // results come from float32 pairs (df32.cuh), and the loops are straight code:
 // sphere grid render 10.70 -> 10.45 ms, room render 3.54 -> 3.44 ms.

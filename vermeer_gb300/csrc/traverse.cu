@@ -631,6 +631,17 @@ __device__ __forceinline__ void load_ray_pd(const RaySoA& rs, uint64_t i, TRay& 
   ray_setup(r);
 }
 
+// Record i of a reordered batch (RaySoA::rec); returns the ray's input index.
+__device__ __forceinline__ uint32_t load_record(const float4* rec, uint64_t i, TRay& r) {
+  const float4 a = __ldg(rec + 2 * i), b = __ldg(rec + 2 * i + 1);
+  r.ox = a.x; r.oy = a.y; r.oz = a.z;
+  r.dx = a.w; r.dy = b.x; r.dz = b.y;
+  r.tclosest = b.z;
+  r.time = 0.0f;
+  ray_setup(r);
+  return __float_as_uint(b.w);
+}
+
 __device__ __forceinline__ void load_ray(const RaySoA& rs, uint64_t i, TRay& r) {
   r.ox = __ldg(rs.px + i); r.oy = __ldg(rs.py + i); r.oz = __ldg(rs.pz + i);
   r.dx = __ldg(rs.dx + i); r.dy = __ldg(rs.dy + i); r.dz = __ldg(rs.dz + i);
@@ -1575,14 +1586,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
         const uint64_t i = base + __popc(need & lanes_below);
         if (i < n) {
           if (!MOTION && rays.rec) {  // the key-ordered copy as records (RaySoA::rec)
-            const float4* A = static_cast<const float4*>(rays.rec);
-            const float4 a = __ldg(A + 2 * i), b = __ldg(A + 2 * i + 1);
-            r.ox = a.x; r.oy = a.y; r.oz = a.z;
-            r.dx = a.w; r.dy = b.x; r.dz = b.y;
-            r.tclosest = b.z;
-            r.time = 0.0f;
-            ray_setup(r);
-            rid = __float_as_uint(b.w);
+            rid = load_record(static_cast<const float4*>(rays.rec), i, r);
           } else {
             rid = order ? (uint64_t)__ldg(order + i) : i;
             load_ray(rays, i, r);
@@ -1843,20 +1847,32 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
     on += (size_t)o * n_nodes;
     return true;
   };
+  // A static scene's reordered rays come as records (RaySoA::rec).
+  const float4* rec = MOT ? nullptr : static_cast<const float4*>(rays.rec);
+  auto input_index = [&]() -> uint64_t {
+    if (rec) return __float_as_uint(__ldg(&rec[2 * li + 1].w));
+    return order ? (uint64_t)__ldg(order + li) : li;
+  };
   auto world_ray = [&]() {  // the ray of the stream, its Tclosest and time kept
     load_ray_pd(rays, li, r);
     slab = slab_ray(r);
   };
   auto sphere = [&](const DMesh& M, uint32_t g) {  // an analytic sphere: tested here, no stack
     TRay w;
-    w.ox = __ldg(rays.px + li); w.oy = __ldg(rays.py + li); w.oz = __ldg(rays.pz + li);
-    w.dx = __ldg(rays.dx + li); w.dy = __ldg(rays.dy + li); w.dz = __ldg(rays.dz + li);
+    if (rec) {
+      const float4 a = __ldg(rec + 2 * li), c = __ldg(rec + 2 * li + 1);
+      w.ox = a.x; w.oy = a.y; w.oz = a.z;
+      w.dx = a.w; w.dy = c.x; w.dz = c.y;
+    } else {
+      w.ox = __ldg(rays.px + li); w.oy = __ldg(rays.py + li); w.oz = __ldg(rays.pz + li);
+      w.dx = __ldg(rays.dx + li); w.dy = __ldg(rays.dy + li); w.dz = __ldg(rays.dz + li);
+    }
     w.tclosest = r.tclosest;
     HitRec h;
     if (!sphere_hit(M, w, h)) return;
     r.tclosest = w.tclosest;
     hit = true;
-    const uint64_t rid = order ? (uint64_t)__ldg(order + li) : li;
+    const uint64_t rid = input_index();
     store_found(hits, rid, 0, 0.0f, 0.0f, 0.0f);
     if (hits.geom) hits.geom[rid] = (int)g;
   };
@@ -1944,7 +1960,8 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
         const uint64_t i = b0 + __popc(idle & lanes_below);
         if (i < n) {
           li = i;
-          load_ray(rays, i, r);
+          if (rec) load_record(rec, i, r);
+          else load_ray(rays, i, r);
           slab = slab_ray(r);
           hit = false;
           node = -1;
@@ -2082,7 +2099,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
       if (any_leaf) {
         need = true;  // the rest of the mesh, then the leaf's next geom or the top level
         if (idx != -1) {
-          const uint64_t rid = order ? (uint64_t)__ldg(order + li) : li;
+          const uint64_t rid = input_index();
           store_found(hits, rid, mot ? __ldg(M->elem + idx) : idx, U, V, W);
           if (hits.geom) hits.geom[rid] = geom;
           hit = true;
@@ -2093,7 +2110,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
     if (alive) {
       if (!walking && !need && node == -1) done = true;
       if (done) {
-        const uint64_t rid = order ? (uint64_t)__ldg(order + li) : li;
+        const uint64_t rid = input_index();
         if (hits.t) hits.t[rid] = r.tclosest;
         if (!hit) {
           store_found(hits, rid, -1, 0.0f, 0.0f, 0.0f);
