@@ -17,3 +17,15 @@ def test_large_and_small_batches_shade_alike(ctx, kind):
     assert st["samples"] == w * h * it
     b, _ = ctx.render_path(w, h, 0, it, 5, max_depth=6, max_batch_samples=w * h * 3)
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("w", [1, 31, 32, 33, 255, 257])
+@pytest.mark.parametrize("kind", ["room", "furnace"])
+def test_queue_remainders(ctx, kind, w):
+    """The hits that wait for a full group: the iterations in one batch, whose
+    rounds leave other remainders than batches of one iteration each."""
+    from vermeer_gb300 import scenes
+    ctx.load_scene(scenes.small_room_ext(300, seed=4) if kind == "room" else scenes.furnace(subdiv=4))
+    a, _ = ctx.render_path(w, 1, 0, 37, 9, max_depth=5)
+    b, _ = ctx.render_path(w, 1, 0, 37, 9, max_depth=5, max_batch_samples=w)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))

@@ -472,13 +472,19 @@ __global__ void __launch_bounds__(kPtBlock) k_pt_prep(PtBatch b, uint32_t d) {
 // So the vertex is a sequence of short phases, the warp together again after
 // each, and the BSDF one piece of code both directions go through.
 //
+// A path that left the scene only adds the environment, so its lane would idle
+// through every phase (12.5 of 32 lanes were active on the sphere grid's first
+// queue).  It ends as it is read; the others' queue indices wait in shared
+// memory until a group (the warp; BIG: the block) is full.  That grid's
+// 8.3M-path render 10.51 -> 9.97 ms, 16 jobs 6.21 -> 6.12 ms.
+//
 // BIG (batches of kPtBigBatch paths or more): a block's warps also wait for each
 // other between phases, so they fetch a phase's instructions once for all, at
-// 4 blocks per SM (64 registers); the sphere grid's 8.3M-path render 11.39 ->
-// 10.72 ms (warps alone 11.28 at 3 blocks, 11.10 at 4).  In a smaller batch a
-// warp waits mostly on its own chain: warps alone at 3 blocks (80 registers),
-// both directions' BSDF inline: 3,072 paths 576 us (590 with BIG), 16 jobs of
-// 131,072 paths 6.32 ms (6.34).
+// 4 blocks per SM (64 registers); 11.39 -> 10.72 ms when it came (warps alone
+// 11.28 at 3 blocks, 11.10 at 4; with the queue 9.97 at 4 blocks, 10.20 at 3).
+// In a smaller batch a warp waits mostly on its own chain: warps alone at 3
+// blocks (80 registers), both directions' BSDF inline: 3,072 paths 576 us (590
+// with BIG), 16 jobs of 131,072 paths 6.32 ms (6.34).
 constexpr uint64_t kPtBigBatch = 1u << 22;
 template <bool BIG>
 __device__ __forceinline__ void phase_end() {
@@ -499,72 +505,104 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : (BIG ? 4 
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const int nL = (int)b.nl;
   const uint32_t base = 8 * d;
-  for (uint64_t r = 0; r < nround; ++r) {
-    const uint64_t i = r * stride + tid;
+  // A path's radiance; TRAIN: the radiance before this vertex closes its previous record.
+  auto radiance = [&](uint32_t p) -> V3 {
+    const V3 L = v3(b.lx[p], b.ly[p], b.lz[p]);
+    if (TRAIN) {
+      const uint32_t lr = b.last_rec[p];
+      if (lr != 0xffffffffu) {
+        b.rec[(size_t)(kRMark + 0) * b.rcap + lr] = L.x;
+        b.rec[(size_t)(kRMark + 1) * b.rcap + lr] = L.y;
+        b.rec[(size_t)(kRMark + 2) * b.rcap + lr] = L.z;
+        b.last_rec[p] = 0xffffffffu;
+      }
+    }
+    return L;
+  };
+  constexpr uint32_t kGroup = BIG ? kPtBlock : 32;
+  __shared__ uint32_t hits[2 * kPtBlock], n_hits;
+  uint32_t* const hq = hits + (BIG ? 0 : 2 * (threadIdx.x & ~31u));
+  const uint32_t rank = BIG ? threadIdx.x : threadIdx.x & 31u;
+  uint32_t held = 0;
+  if (BIG) {
+    if (threadIdx.x == 0) n_hits = 0;
+    __syncthreads();
+  }
+  for (uint64_t r = 0; r <= nround; ++r) {
+    // ---- paths that left the scene end here, the others queue up (the last
+    // round shades what is left)
+    uint64_t i = r * stride + tid;
+    const bool hit = r < nround && i < n && b.hprim[i] >= 0;
+    if (r < nround && i < n && !hit && (TRAIN || b.has_env)) {
+      const uint32_t p = qp[i];
+      const V3 L = radiance(p);
+      if (b.has_env) {
+        const V3 beta = v3(b.bx[p], b.by[p], b.bz[p]), Le = v3(b.env[0], b.env[1], b.env[2]);
+        const float pdf_prev = b.pdf[p];
+        const float w = pdf_prev != 0.0f ? power_w(pdf_prev, b.sel * kInv4Pi) : 1.0f;
+        b.lx[p] = L.x + beta.x * Le.x * w; b.ly[p] = L.y + beta.y * Le.y * w; b.lz[p] = L.z + beta.z * Le.z * w;
+      }
+    }
+    const unsigned hm = __ballot_sync(0xffffffffu, hit);
+    uint32_t at = held;
+    if (BIG) {
+      if ((threadIdx.x & 31u) == 0 && hm != 0u) at = atomicAdd(&n_hits, (uint32_t)__popc(hm));
+      at = __shfl_sync(0xffffffffu, at, 0);
+    }
+    if (hit) hq[at + __popc(hm & ((1u << (threadIdx.x & 31u)) - 1u))] = (uint32_t)i;
+    phase_end<BIG>();
+    held = BIG ? n_hits : held + __popc(hm);
+    const uint32_t take = min(held, kGroup);
+    const bool go = take == kGroup || (r == nround && take > 0);
+    const bool live = go && rank < take;
+    if (live) i = hq[held - take + rank];
+    phase_end<BIG>();
+    if (!go) continue;
+    held -= take;
+    if (BIG && threadIdx.x == 0) n_hits = held;
     uint32_t p = 0, shid = 0;
     uint64_t key = 0;
     bool shade = false;  // the vertex scatters: light sample and continuation
     V3 beta = v3(0, 0, 0), wi = v3(0, 0, 0), org = v3(0, 0, 0);
     Ctx sc;
-    // ---- the hit: attributes, emission or environment with MIS
-    if (i < n) {
+    // ---- the hit: attributes, emission with MIS
+    if (live) {
       p = qp[i];
       const V3 D = v3(q[3 * (size_t)b.cap + i], q[4 * (size_t)b.cap + i], q[5 * (size_t)b.cap + i]);
       beta = v3(b.bx[p], b.by[p], b.bz[p]);
-      V3 L = v3(b.lx[p], b.ly[p], b.lz[p]);
-      if (TRAIN) {  // the radiance before this vertex closes the previous record
-        const uint32_t lr = b.last_rec[p];
-        if (lr != 0xffffffffu) {
-          b.rec[(size_t)(kRMark + 0) * b.rcap + lr] = L.x;
-          b.rec[(size_t)(kRMark + 1) * b.rcap + lr] = L.y;
-          b.rec[(size_t)(kRMark + 2) * b.rcap + lr] = L.z;
-          b.last_rec[p] = 0xffffffffu;
-        }
-      }
+      V3 L = radiance(p);
       const float pdf_prev = b.pdf[p];
       key = b.key[p];
-      const int32_t prim = b.hprim[i];
-      V3 Le = v3(0, 0, 0);
-      float w = 1.0f;  // the MIS weight of what the ray found by itself
-      bool emits = false;
-      if (prim < 0) {
-        if (b.has_env) {
-          emits = true;
-          Le = v3(b.env[0], b.env[1], b.env[2]);
-          if (pdf_prev != 0.0f) w = power_w(pdf_prev, b.sel * kInv4Pi);
+      const int32_t prim = b.hprim[i], geom = b.hgeom[i];
+      const V3 Ro = v3(q[i], q[(size_t)b.cap + i], q[2 * (size_t)b.cap + i]);
+      if (surface_attributes<GROUPS>(b.meshes[geom], prim, b.hu[i], b.hv[i], b.hw[i], Ro, D, b.ht[i],
+                                     q[7 * (size_t)b.cap + i], sc, shid)) {
+        const vmr_shader_std& sh = b.shaders[shid];
+        wi = v3(-D.x, -D.y, -D.z);
+        const bool front = dot(sc.Ng, wi) > 0.0f;
+        const RGB e = emission(sh);
+        const V3 Le = v3(e.c[0], e.c[1], e.c[2]);
+        if (front && (Le.x != 0.0f || Le.y != 0.0f || Le.z != 0.0f)) {
+          float w = 1.0f;  // the MIS weight of what the ray found by itself
+          const int32_t li = (uint32_t)geom < b.n_geoms ? b.light_of_geom[geom] : -1;
+          if (pdf_prev != 0.0f && li >= 0) {
+            const PtLight& l = b.lights[li];
+            const float t = b.ht[i];
+            const float pl = b.sel * (t * t) / (l.area * fabsf(dot(D, sc.Ng)));
+            w = power_w(pdf_prev, pl);
+          }
+          L = add(L, v3(beta.x * Le.x * w, beta.y * Le.y * w, beta.z * Le.z * w));
+          b.lx[p] = L.x; b.ly[p] = L.y; b.lz[p] = L.z;
         }
-      } else {
-        const int32_t geom = b.hgeom[i];
-        const V3 Ro = v3(q[i], q[(size_t)b.cap + i], q[2 * (size_t)b.cap + i]);
-        if (surface_attributes<GROUPS>(b.meshes[geom], prim, b.hu[i], b.hv[i], b.hw[i], Ro, D, b.ht[i],
-                                       q[7 * (size_t)b.cap + i], sc, shid)) {
-          const vmr_shader_std& sh = b.shaders[shid];
-          wi = v3(-D.x, -D.y, -D.z);
-          const bool front = dot(sc.Ng, wi) > 0.0f;
-          const RGB e = emission(sh);
-          Le = v3(e.c[0], e.c[1], e.c[2]);
-          if (front && (Le.x != 0.0f || Le.y != 0.0f || Le.z != 0.0f)) {
-            emits = true;
-            const int32_t li = (uint32_t)geom < b.n_geoms ? b.light_of_geom[geom] : -1;
-            if (pdf_prev != 0.0f && li >= 0) {
-              const PtLight& l = b.lights[li];
-              const float t = b.ht[i];
-              const float pl = b.sel * (t * t) / (l.area * fabsf(dot(D, sc.Ng)));
-              w = power_w(pdf_prev, pl);
-            }
-          }
-          const float tw = ((sh.flags & VMR_SH_DIFFUSE_STRENGTH) ? sh.diffuse_strength : 0.0f) +
-                           ((sh.flags & VMR_SH_SPEC1_STRENGTH) ? sh.spec1_strength : 0.0f);
-          shade = d < b.max_depth && tw != 0.0f;
-          if (!front) {  // two-sided: face the incoming ray
-            sc.N = v3(-sc.N.x, -sc.N.y, -sc.N.z);
-            sc.Ng = v3(-sc.Ng.x, -sc.Ng.y, -sc.Ng.z);
-            sc.Poffset = v3(-sc.Poffset.x, -sc.Poffset.y, -sc.Poffset.z);
-          }
+        const float tw = ((sh.flags & VMR_SH_DIFFUSE_STRENGTH) ? sh.diffuse_strength : 0.0f) +
+                         ((sh.flags & VMR_SH_SPEC1_STRENGTH) ? sh.spec1_strength : 0.0f);
+        shade = d < b.max_depth && tw != 0.0f;
+        if (!front) {  // two-sided: face the incoming ray
+          sc.N = v3(-sc.N.x, -sc.N.y, -sc.N.z);
+          sc.Ng = v3(-sc.Ng.x, -sc.Ng.y, -sc.Ng.z);
+          sc.Poffset = v3(-sc.Poffset.x, -sc.Poffset.y, -sc.Poffset.z);
         }
       }
-      if (emits) L = add(L, v3(beta.x * Le.x * w, beta.y * Le.y * w, beta.z * Le.z * w));
-      b.lx[p] = L.x; b.ly[p] = L.y; b.lz[p] = L.z;
     }
     phase_end<BIG>();
     // ---- the shading frame and the material
@@ -718,7 +756,7 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : (BIG ? 4 
       phase_end<BIG>();
     }
     const float so[3] = {org.x, org.y, org.z};
-    const float time = i < n ? q[7 * (size_t)b.cap + i] : 0.0f;
+    const float time = live ? q[7 * (size_t)b.cap + i] : 0.0f;
     if (cont) {
       b.pdf[p] = delta ? 0.0f : rQ;
       b.bx[p] = beta.x; b.by[p] = beta.y; b.bz[p] = beta.z;
