@@ -110,6 +110,10 @@ struct PtBatch {
   float* qray[2];        // 8 * cap floats: px py pz dx dy dz tmax time
   uint32_t* qpath[2];
   int32_t *hprim, *hgeom;
+  // The flattened scene's leaf positions (PtFlat): geoms, then the geoms' leaf
+  // positions, n_prims each; null: the trace wrote the scene's ids.
+  const uint32_t* flat_map;
+  uint32_t n_prims;      // hits are below it (2^31 without the map)
   float *ht, *hu, *hv, *hw;
   // shadow queue
   float* sray;           // 8 * cap
@@ -390,6 +394,19 @@ __device__ V3 gmix_sample(const GMix& g, float u, float u1, float u2) {
                       w * mu.z + st * (cp * t1.z + sp * t2.z)));
 }
 
+// The geom and its leaf position of queue entry i, a hit.  (A pass of its own
+// over the queue after each trace took 79 us of the sphere grid's 9.97 ms and a
+// launch a bounce.)
+__device__ __forceinline__ void scene_hit(const PtBatch& b, uint64_t i, int32_t& prim, int32_t& geom) {
+  prim = b.hprim[i];
+  if (b.flat_map) {
+    geom = (int32_t)__ldg(b.flat_map + prim);
+    prim = (int32_t)__ldg(b.flat_map + b.n_prims + prim);
+  } else {
+    geom = b.hgeom[i];
+  }
+}
+
 // CKEYS: the camera has motion keys (b.cam_nkeys >= 2).
 template <bool CKEYS>
 __global__ void __launch_bounds__(kPtBlock) k_pt_generate(PtBatch b) {
@@ -437,13 +454,14 @@ __global__ void __launch_bounds__(kPtBlock) k_pt_prep(PtBatch b, uint32_t d) {
   const float* q = b.qray[d & 1];
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     V3 P = v3(b.glo[0], b.glo[1], b.glo[2]), N = v3(0, 0, 1), wi = v3(0, 0, 1);
-    const int32_t prim = b.hprim[i];
-    if (prim >= 0) {
+    if ((uint32_t)b.hprim[i] < b.n_prims) {
       Ctx sc;
       uint32_t shid = 0;
+      int32_t prim, geom;
+      scene_hit(b, i, prim, geom);
       const V3 Ro = v3(q[i], q[(size_t)b.cap + i], q[2 * (size_t)b.cap + i]);
       const V3 Rd = v3(q[3 * (size_t)b.cap + i], q[4 * (size_t)b.cap + i], q[5 * (size_t)b.cap + i]);
-      if (surface_attributes<GROUPS>(b.meshes[b.hgeom[i]], prim, b.hu[i], b.hv[i], b.hw[i], Ro, Rd, b.ht[i],
+      if (surface_attributes<GROUPS>(b.meshes[geom], prim, b.hu[i], b.hv[i], b.hw[i], Ro, Rd, b.ht[i],
                              q[7 * (size_t)b.cap + i], sc, shid)) {
         wi = v3(-q[3 * (size_t)b.cap + i], -q[4 * (size_t)b.cap + i], -q[5 * (size_t)b.cap + i]);
         P = sc.P;
@@ -532,7 +550,7 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : (BIG ? 4 
     // ---- paths that left the scene end here, the others queue up (the last
     // round shades what is left)
     uint64_t i = r * stride + tid;
-    const bool hit = r < nround && i < n && b.hprim[i] >= 0;
+    const bool hit = r < nround && i < n && (uint32_t)b.hprim[i] < b.n_prims;
     if (r < nround && i < n && !hit && (TRAIN || b.has_env)) {
       const uint32_t p = qp[i];
       const V3 L = radiance(p);
@@ -573,7 +591,8 @@ __global__ void __launch_bounds__(kPtBlock, GROUPS ? 1 : (GUIDED ? 2 : (BIG ? 4 
       V3 L = radiance(p);
       const float pdf_prev = b.pdf[p];
       key = b.key[p];
-      const int32_t prim = b.hprim[i], geom = b.hgeom[i];
+      int32_t prim, geom;
+      scene_hit(b, i, prim, geom);
       const V3 Ro = v3(q[i], q[(size_t)b.cap + i], q[2 * (size_t)b.cap + i]);
       if (surface_attributes<GROUPS>(b.meshes[geom], prim, b.hu[i], b.hv[i], b.hw[i], Ro, D, b.ht[i],
                                      q[7 * (size_t)b.cap + i], sc, shid)) {
@@ -970,29 +989,12 @@ struct PtSort {
 
 // The flattened scene (vmr::flat_scene) the bounce loop traces instead of
 // the two-level scene: one mesh over every triangle, its hits mapped back to
-// (geom, the geom's leaf position) by k_flat_remap.
+// (geom, the geom's leaf position) where they are read (scene_hit).
 struct PtFlat {
   const DMesh* mesh = nullptr;
   const uint32_t* map = nullptr;  // [2 * n]: geom, then the geom's leaf position
   uint32_t n = 0;
 };
-
-// Closest hits of a flattened-scene trace back to the scene's ids: the flat
-// mesh's leaf position e becomes geom map[e] and triangle map[n + e].
-__global__ void __launch_bounds__(kPtBlock) k_flat_remap(const uint32_t* __restrict__ map, uint32_t n,
-                                                          int32_t* prim, int32_t* geom,
-                                                          const unsigned long long* qlen, uint64_t cap) {
-  const uint64_t m = *qlen < cap ? *qlen : cap;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-    const int32_t e = prim[i];
-    if (e >= 0 && (uint32_t)e < n) {
-      geom[i] = (int32_t)__ldg(map + e);
-      prim[i] = (int32_t)__ldg(map + n + e);
-    } else {
-      geom[i] = -1;
-    }
-  }
-}
 
 int launch_batch(vmr_ctx* ctx, const PtBatch& b, const DTop& top, DScratch* scr, int grid, bool guided, bool train,
                  const guide::GuideRows& grows, const PtSort& srt, const PtFlat& flat) {
@@ -1036,8 +1038,6 @@ int launch_batch(vmr_ctx* ctx, const PtBatch& b, const DTop& top, DScratch* scr,
     if (srt.on && d > 0 && sort_queue(l) != 0) return pfail(ctx, VMR_ERR_CUDA, "ray sort launch failed");
     if (flat.mesh) {
       if (launch_trace_mesh(*flat.mesh, l) != 0) return pfail(ctx, VMR_ERR_CUDA, "trace launch failed");
-      k_flat_remap<<<grid, kPtBlock, 0, st>>>(flat.map, flat.n, b.hprim, b.hgeom, &b.qlen[d], b.cap);
-      PCUDA(cudaGetLastError());
     } else if (launch_trace_scene(top, l) != 0) {
       return pfail(ctx, VMR_ERR_CUDA, "trace launch failed");
     }
@@ -1406,6 +1406,8 @@ static int render_path_impl(vmr_ctx* ctx, const vmr_path_params* p, float* fb, v
     flat.mesh = flat_scene(ctx, &flat.map, &flat.n, &fs);
     if (fs != VMR_OK) return fs;
   }
+  b.flat_map = flat.mesh ? flat.map : nullptr;
+  b.n_prims = flat.mesh ? flat.n : 1u << 31;
   PtSort srt;
   if (sort_on) {
     srt.on = true;
