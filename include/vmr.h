@@ -416,7 +416,7 @@ typedef struct {
 enum {
     /* The shading's transcendentals (light and BSDF sampling, Oren-Nayar,
      * the spherical-triangle sampling) in float32 instead of the reference's
-     * float64-rounded-to-float32 (math/sincos.go): off the FP64 pipe, no
+     * float64-rounded-to-float32 (math/sincos.go): fewer instructions, no
      * longer bit-exact with the oracle; the image stays within the stated
      * tolerance of the float64 one. */
     VMR_RENDER_F32 = 1
@@ -783,7 +783,7 @@ int vmr_guide_train_step(vmr_ctx* ctx, const float* pos, const float* nrm, const
  * loop): the same trace as vmr_trace_mesh with device pointers (the mesh's
  * own tuning, autotuned or the context's), but every scratch buffer (work
  * counter, status word, ray-reordering buffers) lives in one static device
- * array of about 11 MB that stays on the GPU until the process exits.
+ * array of about 12 MB that stays on the GPU until the process exits.
  * vmr_create resolves that array on its device (this is where the array is
  * loaded onto the GPU); the call itself allocates nothing.
  *   - flags must hold VMR_TRACE_DEVICE (rays and hits are device or managed

@@ -172,7 +172,7 @@ constexpr int kSharedStackEntries = 16;
 // b = 3..5, x the octant of the class's other two signs for b <= 4.
 constexpr int kSortMaxBits = 5;
 constexpr int kSortOctantBits = 4;
-constexpr int kSortBucketsMax = 6 << (3 * kSortMaxBits);
+constexpr int kSortBucketsMax = 2 * (6 << (3 * kSortMaxBits));  // the histogram, then its scan
 constexpr uint32_t sort_buckets(int bits) { return (6u << (3 * bits)) * (bits <= kSortOctantBits ? 4u : 1u); }
 // The width a tuning of 0 takes: 16^3 cells, or 8^3 for batches in which that
 // many buckets (98,304) would hold a few rays each and their scan costs more
