@@ -52,9 +52,9 @@ __device__ __forceinline__ float gatan(float x) { return atan_rn(x); }
 __device__ __forceinline__ float gatan2(float y, float x) { return (float)atan2((double)y, (double)x); }
 __device__ __forceinline__ float gacos(float x) { return acos_rn(x > 1.0f ? 1.0f : (x < -1.0f ? -1.0f : x)); }
 // The same functions under the reference-mode precision switch: F32 false
-// is the float64 evaluation above (the reference's math/sincos.go, bit for
+// is float64's result rounded, as above (the reference's math/sincos.go, bit for
 // bit with the oracle); F32 true is CUDA's float32 functions (within 2 ulp),
-// the VMR_RENDER_F32 option, which keeps the shading off the FP64 pipe.
+// the VMR_RENDER_F32 option, which takes fewer instructions.
 template <bool F32> __device__ __forceinline__ float msin(float x) { return F32 ? sinf(x) : gsin(x); }
 template <bool F32> __device__ __forceinline__ float mcos(float x) { return F32 ? cosf(x) : gcos(x); }
 template <bool F32> __device__ __forceinline__ void msincos(float x, float& s, float& c) {

@@ -2328,8 +2328,8 @@ int launch_persistent(K k, const TraceLaunch& l, int block, A... args) {
 }
 
 // tuning.kernel: bit 0 = while-while (else step-scheduled), bit 1 = L1
-// prefetch of the next node, bit 2 = 64-register cap (while-while, 128
-// threads, 8 resident blocks), bit 3 = ray reordering (host side).
+// prefetch of the next node, bit 2 = register cap (while-while, 128 threads; 7
+// resident blocks, 5 for motion), bit 3 = ray reordering (host side).
 template <class K, class... A>
 int launch_persistent_smem(K k, const TraceLaunch& l, int block, size_t smem, A... args) {
   int dev = 0, sms = 0, per_sm = 0;
