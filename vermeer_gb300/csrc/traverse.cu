@@ -1536,7 +1536,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
   __shared__ int2 leaf_map[COOP ? (MINB > 0 ? 128 : 256) : 1];
   // A shadow ray's Tclosest holds until its traversal ends, and what was pushed was
   // not behind it: nothing is culled at a pop, and its 4-byte entries halve the
-  // stack's L1 traffic (600,011 rays 477 -> 467 us).
+  // stack's L1 traffic (300,007 rays 477 -> 467 us).
   SplitStack<SS, !ANY> stk;
   if (SS > 0) {
     stk.stride = blockDim.x;
@@ -2367,10 +2367,10 @@ int launch_mesh_t(const DMesh& mesh, const TraceLaunch& l) {
   const int v = l.kernel;
   if (v & kKernelWhileWhile) {
     // the register cap: 7 resident blocks per SM (72 registers) for static
-    // meshes (with the record fetch, 8 blocks at 64 registers spilled 108 B
-    // and ran 5% slower); motion meshes hold both keys' boxes and vertices
-    // and run fastest at 5 blocks (96 registers: 130 against 100 Mrays/s
-    // at 8)
+    // meshes (4,194,304 rays: 8 blocks 4% slower, 9 9%; 300,007 shadow rays 465
+    // us, 6 and 8 blocks 484, 9 610); motion meshes hold both keys' boxes and
+    // vertices and run fastest at 5 blocks (96 registers: 262,147 rays 1.35 ms,
+    // 4 blocks 1.44, 6 1.57)
     if (v & kKernelRegCap) return launch_ww<MOTION, ANY, COUNT, MOTION ? 5 : 7>(mesh, l, 128);
     return launch_ww<MOTION, ANY, COUNT, 0>(mesh, l, block);
   }
