@@ -1,0 +1,78 @@
+"""Rays whose time a motion mesh has no keys for.
+
+A mesh is a miss for such a ray and the rest of the scene is not: the
+while-while scene kernel against the single-loop kernel (tuning kernel 0), bit
+for bit.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+OUT = ("prim", "t", "u", "v", "w")
+OUTSIDE = (-0.25, -1e-30, np.nextafter(np.float32(1), np.float32(2)), 1.5, 7.0, np.inf, -np.inf)
+
+
+def _rays(n, seed, times):
+    """Times inside the keys, and each of times at every third ray in turn."""
+    from vermeer_gb300 import scenes
+    r = scenes.incoherent_rays(n, seed)
+    r[:, 7] = scenes.uniform(seed, n, 77).astype(np.float32)
+    at = np.arange(0, n, 3)
+    r[at, 7] = np.asarray(times, np.float32)[(at // 3) % len(times)]
+    return r
+
+
+def _equal_to_kernel_0(ctx, trace, outputs):
+    got = {}
+    try:
+        for shadow in (False, True):
+            for k in (0, 13, 45):
+                ctx.set_tuning(kernel=k)
+                got[shadow, k] = trace(shadow)
+            for k in (13, 45):
+                for o in outputs:
+                    x, y = (z[o].view(np.uint32) if z[o].dtype == np.float32 else z[o]
+                            for z in (got[shadow, k], got[shadow, 0]))
+                    bad = np.nonzero(x != y)[0]
+                    assert bad.size == 0, (o, k, shadow, bad.size, bad[:4])
+    finally:
+        ctx.set_tuning()
+    return got[False, 45]
+
+
+def _static_top_over_moving_meshes(ctx, n_geoms, tris, keys):
+    """A static top level uploaded over meshes of which two in three move (of
+    those one in two has a transform as well) and a sphere: the top level of the
+    meshes as they are at the first key."""
+    from vermeer_gb300 import scenes
+    still, geoms = [], []
+    rng = np.random.default_rng(23)
+    for k in range(n_geoms):
+        v, ip = scenes.triangle_soup(tris + 40 * k, 80 + k, lo=0.1 * (k % 7), hi=0.1 * (k % 7) + 0.4, edge=0.06)
+        still.append(ctx.mesh_build(v, ip))
+        if k % 3 == 0:
+            geoms.append(still[-1])
+            continue
+        step = np.float32(0.02) * rng.standard_normal(3).astype(np.float32)
+        geoms.append(ctx.mesh_build(np.concatenate([v + np.float32(q) * step for q in range(keys)]), ip, keys=keys,
+                                    motion_mode=1))
+        if k % 3 == 2:
+            ctx.mesh_set_transform(geoms[-1], [1, 0.02, 0, 0, -0.02, 1, 0, 0, 0, 0, 1, 0, 0.01, 0, 0.02, 1])
+    still.append(ctx.sphere_add((0.4, 0.5, 0.6), 0.15))
+    geoms.append(still[-1])
+    ctx.scene_build(still)
+    e = ctx.scene_export(len(still))
+    assert e["keys"] == 1
+    moved = dict(zip(still, geoms))
+    ctx.scene_upload(np.array([moved[g] for g in e["geom_order"]], np.uint32), nodes=e["nodes"])
+    return geoms
+
+
+@pytest.mark.parametrize("n_geoms,tris", [(2, 20), (9, 200), (40, 60)])
+@pytest.mark.parametrize("keys", [2, 3])
+def test_static_top_level_over_moving_meshes(ctx, n_geoms, tris, keys):
+    geoms = _static_top_over_moving_meshes(ctx, n_geoms, tris, keys)
+    rays = _rays(8191, 41, OUTSIDE)
+    r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
+    still = np.isin(r["geom"], [g for k, g in enumerate(geoms) if k % 3 == 0 or k == n_geoms] + [-1])
+    assert still[::3].all() and not still.all()

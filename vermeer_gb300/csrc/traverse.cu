@@ -1824,15 +1824,21 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
   float tm = 0.f;
   bool mxf = false;  // the current mesh has a transform: r is its object-space ray
 
-  // The level of a static (keys 1) or motion tree; false outside its keys.
+  // The level of a static (keys 1) or motion tree; false outside its keys, and
+  // then the lane stays in the level it is in (a top-level leaf's next geom, or
+  // the top level's next entry, follows).
   auto enter = [&](const ONode* onodes, uint32_t n_nodes, uint32_t keys) -> bool {
+    float t = 0.f;
+    int key = 0, key2 = 0;
+    if (MOT && keys > 1) {
+      float omt;
+      if (!motion_keys(keys, r.time, t, omt, key, key2)) return false;
+    }
     on = onodes;
     level = r.exact || !onodes ? kLevelNodes : kLevelStatic;
     uint32_t o = r.oct;
     if (MOT && keys > 1) {
-      float omt;
-      int key, key2;
-      if (!motion_keys(keys, r.time, tm, omt, key, key2)) return false;
+      tm = t;
       dkey = key2 != key ? n_nodes : 0u;
       o = o * keys + (uint32_t)key;
       if (level == kLevelStatic) level = kLevelMotion;
