@@ -1,8 +1,8 @@
-"""Rays whose time a motion mesh has no keys for.
+"""Rays whose time a motion mesh has no keys for, or is not a number.
 
 A mesh is a miss for such a ray and the rest of the scene is not: the
-while-while scene kernel against the single-loop kernel (tuning kernel 0), bit
-for bit.
+while-while kernels against the step-scheduled mesh kernel and the single-loop
+scene kernel (tuning kernel 0), bit for bit.
 """
 import numpy as np
 import pytest
@@ -76,3 +76,30 @@ def test_static_top_level_over_moving_meshes(ctx, n_geoms, tris, keys):
     r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
     still = np.isin(r["geom"], [g for k, g in enumerate(geoms) if k % 3 == 0 or k == n_geoms] + [-1])
     assert still[::3].all() and not still.all()
+
+
+@pytest.mark.parametrize("n_geoms,tris", [(2, 20), (9, 200)])
+def test_nan_time_under_a_static_top_level(ctx, n_geoms, tris):
+    geoms = _static_top_over_moving_meshes(ctx, n_geoms, tris, 2)
+    rays = _rays(4099, 43, (np.nan,))
+    r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
+    still = np.isin(r["geom"], [g for k, g in enumerate(geoms) if k % 3 == 0 or k == n_geoms] + [-1])
+    assert still[::3].all() and not still.all()
+
+
+@pytest.mark.parametrize("keys", [2, 3])
+@pytest.mark.parametrize("tris", [1, 17, 1500])
+def test_times_without_keys_miss_a_motion_mesh(ctx, keys, tris):
+    from vermeer_gb300 import scenes
+    v, ip = scenes.triangle_soup(tris, 11, edge=0.2 if tris < 100 else 0.06)
+    step = np.float32(0.05) * scenes.unit_sphere(5, v.shape[0], 3).astype(np.float32)
+    g = ctx.mesh_build(np.concatenate([v + np.float32(q) * step for q in range(keys)]), ip, keys=keys, motion_mode=1)
+    rays = _rays(4099, 47, OUTSIDE + (np.nan,))
+    r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_mesh(g, rays, shadow=shadow), OUT)
+    assert (r["prim"][::3] == -1).all() and ((r["prim"] >= 0).any() or tris == 1)
+    # the same mesh under a top level that moves with it, and one that is still
+    # beside it: nothing of such a scene is met
+    w, iw = scenes.triangle_soup(40, 12, edge=0.2)
+    ctx.scene_build([g, ctx.mesh_build(w, iw)])
+    r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
+    assert (r["geom"][::3] == -1).all() and ((r["geom"] >= 0).any() or tris == 1)

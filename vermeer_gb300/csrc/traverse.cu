@@ -1597,8 +1597,9 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             tm = __fsub_rn(k, fk);
             omt = __fsub_rn(1.0f, tm);
             const int key = (int)fk, key2 = (int)ceilf(k);
-            if (key < 0 || key2 >= (int)m.keys) {
-              // out of the key range: the reference indexes out of bounds; miss
+            if (!(k >= 0.0f) || key2 >= (int)m.keys) {
+              // out of the key range (the reference indexes out of bounds) or a
+              // NaN time (its boxes are NaN, which no ray meets): miss
               store_end(hits, rid, r.tclosest, false);
               alive = false;
             } else {
@@ -1767,7 +1768,9 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
 // visits, pops, culls and triangle tests per ray are the reference's.
 // The key pair and lerp weight of a motion mesh at the ray's time
 // (builtin/geom/polymesh/trace.go:79-84); false outside the key range (the
-// reference would index out of bounds: a miss, as the mesh kernels treat it).
+// reference would index out of bounds: a miss, as the mesh kernels treat it) and
+// for a NaN time, whose lerped boxes no ray meets.  Those tests are on k: the
+// integer of a NaN is 0, and slot_hit passes over a NaN plane.
 __device__ __forceinline__ bool motion_keys(uint32_t keys, float time, float& tm, float& omt, int& key, int& key2) {
   const float k = __fmul_rn(time, (float)(keys - 1));
   const float fk = floorf(k);
@@ -1775,7 +1778,7 @@ __device__ __forceinline__ bool motion_keys(uint32_t keys, float time, float& tm
   omt = __fsub_rn(1.0f, tm);
   key = (int)fk;
   key2 = (int)ceilf(k);
-  return !(key < 0 || key2 >= (int)keys);
+  return k >= 0.0f && key2 < (int)keys;
 }
 
 // The walk is k_trace_mesh_ww's: octant copies of the current level's nodes,
