@@ -1,4 +1,5 @@
-"""Rays whose time a motion mesh has no keys for, or is not a number.
+"""Rays whose time a motion mesh has no keys for, or is not a number, and boxes
+that are not finite at a key.
 
 A mesh is a miss for such a ray and the rest of the scene is not: the
 while-while kernels against the step-scheduled mesh kernel and the single-loop
@@ -103,3 +104,42 @@ def test_times_without_keys_miss_a_motion_mesh(ctx, keys, tris):
     ctx.scene_build([g, ctx.mesh_build(w, iw)])
     r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
     assert (r["geom"][::3] == -1).all() and ((r["geom"] >= 0).any() or tris == 1)
+
+
+def _reach_to_infinity(boxes, kind):
+    """Planes at infinity, on one side or both, along one axis or all, in every
+    third node (boxes: [keys, nodes, 24], min planes of the four children by axis,
+    then max planes)."""
+    b = boxes[:, ::3]
+    axes = range(3) if kind.startswith("all") else (1,)
+    for a in axes:
+        if kind.endswith("below") or kind.endswith("both"):
+            b[..., 4 * a:4 * a + 4] = -np.inf
+        if kind.endswith("above") or kind.endswith("both"):
+            b[..., 12 + 4 * a:16 + 4 * a] = np.inf
+    return boxes
+
+
+@pytest.mark.parametrize("kind", ["one_below", "one_above", "one_both", "all_below", "all_above", "all_both"])
+@pytest.mark.parametrize("keys", [2, 3])
+@pytest.mark.parametrize("tris", [3, 17, 1500])
+def test_motion_boxes_at_infinity(ctx, kind, keys, tris):
+    """At a key such a plane lerps to 0 * inf, a NaN: the slab test must take
+    the box's other plane for it, as the node walk does."""
+    from vermeer_gb300 import scenes
+    v, ip = scenes.triangle_soup(tris, 11, edge=0.2 if tris < 100 else 0.06)
+    step = np.float32(0.05) * scenes.unit_sphere(5, v.shape[0], 3).astype(np.float32)
+    v = np.concatenate([v + np.float32(q) * step for q in range(keys)])
+    e = ctx.mesh_export(ctx.mesh_build(v, ip, keys=keys, motion_mode=1))
+    boxes = _reach_to_infinity(e["mboxes"].copy().reshape(keys, -1, 24), kind)
+    g = ctx.mesh_upload(v, e["idxp"], e["accel_idx"], mnodes=e["mnodes"], mboxes=boxes, bounds=e["bounds"], keys=keys,
+                        motion_mode=1)
+    rays = _rays(4099, 53, (0.0, 1.0, 0.5, 0.25))
+    _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_mesh(g, rays, shadow=shadow), OUT)
+    w, iw = scenes.triangle_soup(40, 12, edge=0.2)
+    ctx.scene_build([g, ctx.mesh_build(w, iw)])
+    t = ctx.scene_export(2)
+    assert t["keys"] == keys
+    ctx.scene_upload(t["geom_order"], mnodes=t["mnodes"],
+                     mboxes=_reach_to_infinity(t["mboxes"].copy().reshape(keys, -1, 24), kind), keys=keys)
+    _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))

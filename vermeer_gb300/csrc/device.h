@@ -219,8 +219,8 @@ int launch_trace_scene(const DTop& top, const TraceLaunch& l);
 // out[8][n]: the octant copies of n nodes (traverse.cu).
 int launch_octant_nodes(const GNode* nodes, uint32_t n, ONode* out, void* stream);
 // out[8][keys][n] of n motion nodes; *bad is set when a box has its planes out
-// of order or a NaN, where lerped near and far planes would not be the lerped
-// boxes' (such a mesh keeps to its mnodes).
+// of order, a NaN or an infinity (0 * inf at a key is a NaN), where lerped near
+// and far planes would not be the lerped boxes' (such a mesh keeps to its mnodes).
 int launch_octant_mnodes(const MNode* nodes, const void* mboxes, uint32_t keys, uint32_t n, ONode* out, int* bad,
                          void* stream);
 int device_sm_count();

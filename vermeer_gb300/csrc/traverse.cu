@@ -1086,7 +1086,7 @@ __global__ void k_octant_mnodes(const MNode* __restrict__ nodes, const float* __
       for (int a = 0; a < 3; ++a) {
         const float mn = box[c + 4 * a], mx = box[12 + c + 4 * a];
         const bool neg = (o >> a) & 1u;
-        if (N.child[c] != kEmptyChild && !(mn <= mx)) *bad = 1;
+        if (N.child[c] != kEmptyChild && !(mn <= mx && isfinite(mn) && isfinite(mx))) *bad = 1;
         r.slot[slot][at_near[a]] = neg ? mx : mn;
         r.slot[slot][at_far[a]] = neg ? mn : mx;
       }
