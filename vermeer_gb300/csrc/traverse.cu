@@ -1530,8 +1530,13 @@ __device__ __forceinline__ int32_t coop_leaf_dispatch(int2* map, const float4* t
   return coop_leaf<-1>(map, tris, lower, r, has, first, count, U, V, W);
 }
 
+// MINB 0 (no register cap asked for): up to 256 threads a block.  The static
+// kernels that scan their leaves lane by lane are held to 3 such blocks per SM (80
+// registers; left alone they took 84 to 90 and lost a block: 1,048,576 rays on
+// 200,003 triangles at 256 threads 2.59 -> 2.09 ms, at 128 threads 2.29 -> 2.04);
+// the others were at 2 with any count up to 128.
 template <bool MOTION, bool ANY, bool COUNT, bool PF, int MINB, int SS, bool COOP = false>
-__global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
+__global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTION || COUNT || COOP ? 1 : 3))
     k_trace_mesh_ww(const DMesh m, RaySoA rays, HitSoA hits, uint64_t n, DScratch* scratch, const uint32_t* order,
                     int walk_tail, const unsigned long long* n_dev) {
   if (n_dev) n = *n_dev < n ? *n_dev : n;  // a wavefront queue's length
