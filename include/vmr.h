@@ -82,7 +82,8 @@ typedef struct {
                             this many lanes still walk and a lane holds a
                             leaf for the cooperative scan (any leaf with bit
                             5, a static leaf without it), 0..31 (default 8;
-                            0 = wait for every lane) */
+                            0 = wait for every lane); at most a quarter of
+                            the rays a warp holds, so 9..31 act as 8 */
     int sort_bits;       /* sort-key width: the ray reordering groups origins
                             in (2^b)^3 cells, b = 3, 4 or 5 (0: 3 for
                             batches below 700,000 rays, else 4) */
