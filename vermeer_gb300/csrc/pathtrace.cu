@@ -1411,7 +1411,7 @@ static int render_path_impl(vmr_ctx* ctx, const vmr_path_params* p, float* fb, v
   PtSort srt;
   if (sort_on) {
     srt.on = true;
-    srt.bits = ctx->tuning.sort_bits ? ctx->tuning.sort_bits : 4;
+    srt.bits = ctx->tuning.sort_bits ? ctx->tuning.sort_bits : default_sort_bits(cap);
     for (int k = 0; k < 3; ++k) {
       srt.bounds[k] = glo[k];
       srt.bounds[3 + k] = ghi[k];
