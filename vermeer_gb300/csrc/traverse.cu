@@ -1146,7 +1146,7 @@ __global__ void k_octant_nodes(const GNode* __restrict__ nodes, uint32_t n, ONod
 template <int SS, bool TS>
 struct SplitStack {
   int* sn;     // shared node ids: entry k of this thread at sn[k * stride]
-  float* st;   // shared T values
+  float* st;   // shared T values (TS)
   int stride;  // threads per block
   using Entry = typename std::conditional<TS, int2, int>::type;
   Entry loc[kStackCapacity - SS];
@@ -1553,7 +1553,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
   if (SS > 0) {
     stk.stride = blockDim.x;
     stk.sn = stack_smem + threadIdx.x;
-    stk.st = reinterpret_cast<float*>(stack_smem + SS * blockDim.x) + threadIdx.x;
+    if (!ANY) stk.st = reinterpret_cast<float*>(stack_smem + SS * blockDim.x) + threadIdx.x;
   }
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanes_below = (1u << lane) - 1u;
@@ -2372,9 +2372,9 @@ int launch_ww(const DMesh& mesh, const TraceLaunch& l, int block) {
     return launch_persistent(k_trace_mesh_ww<MOTION, ANY, COUNT, false, MINB, 0, true>, l, block, mesh, l.rays, l.hits,
                              l.n, l.scratch, l.order, tail, l.n_dev);
   if (l.kernel & kKernelSharedStack) {
-    constexpr int SS = kSharedStackEntries;
+    constexpr int SS = kSharedStackEntries;  // of 4 bytes (any hit: nodes) or 8 (SplitStack)
     return launch_persistent_smem(k_trace_mesh_ww<MOTION, ANY, COUNT, false, MINB, SS>, l, block,
-                                  (size_t)SS * block * 8, mesh, l.rays, l.hits, l.n, l.scratch, l.order, tail, l.n_dev);
+                                  (size_t)SS * block * (ANY ? 4 : 8), mesh, l.rays, l.hits, l.n, l.scratch, l.order, tail, l.n_dev);
   }
   if (l.kernel & kKernelPrefetch)
     return launch_persistent(k_trace_mesh_ww<MOTION, ANY, COUNT, true, MINB, 0>, l, block, mesh, l.rays, l.hits, l.n,
