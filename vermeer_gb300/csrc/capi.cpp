@@ -122,39 +122,61 @@ void fill_xf(const MeshRec& rec, DMesh& d) {
   d.xf_keys = keyed ? rec.dxkeys.as<vmr::anim::Decomp>() : nullptr;
 }
 
-// The octant copies of n nodes.  They only save work: without the memory for
-// them the traces walk the nodes themselves.
-cudaError_t octant_nodes(vmr_ctx* ctx, const DevBuf& nodes, uint32_t n, DevBuf& buf, const vmr::ONode*& out) {
-  out = nullptr;
-  if (n == 0) return cudaSuccess;
-  cudaError_t e = buf.ensure((size_t)8 * n * sizeof(vmr::ONode));
+// Room for bytes of octant copies in buf; got false: there is none, or none to
+// spare (octant_room), and the traces walk the nodes themselves, which gives the
+// same hits.
+constexpr uint64_t kOctantAsk = 1ull << 30;  // fewer bytes are no sixteenth of a device worth asking for
+cudaError_t octant_alloc(vmr_ctx* ctx, size_t bytes, vmr::OctantBuf& buf, bool& got) {
+  got = bytes <= buf.buf.bytes;
+  if (got) return cudaSuccess;
+  const uint64_t held = ctx->octant_bytes - buf.buf.bytes;  // without what this buffer holds now
+  if (held + bytes > kOctantAsk) {
+    if (ctx->device_bytes == 0) {
+      size_t free = 0, total = 0;
+      const cudaError_t e = cudaMemGetInfo(&free, &total);
+      if (e != cudaSuccess) return e;
+      ctx->device_bytes = total;
+    }
+    if (!vmr::octant_room(held, bytes, ctx->device_bytes)) {
+      buf.drop();
+      return cudaSuccess;
+    }
+  }
+  const cudaError_t e = buf.ensure(bytes, &ctx->octant_bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return cudaSuccess;
   }
-  if (e != cudaSuccess) return e;
-  e = (cudaError_t)vmr::launch_octant_nodes(nodes.as<GNode>(), n, buf.as<vmr::ONode>(), ctx->stream);
-  if (e == cudaSuccess) out = buf.as<vmr::ONode>();
+  got = e == cudaSuccess;
+  return e;
+}
+
+// The octant copies of n nodes.
+cudaError_t octant_nodes(vmr_ctx* ctx, const DevBuf& nodes, uint32_t n, vmr::OctantBuf& buf, const vmr::ONode*& out) {
+  out = nullptr;
+  if (n == 0) return cudaSuccess;
+  bool got = false;
+  cudaError_t e = octant_alloc(ctx, (size_t)8 * n * sizeof(vmr::ONode), buf, got);
+  if (e != cudaSuccess || !got) return e;
+  e = (cudaError_t)vmr::launch_octant_nodes(nodes.as<GNode>(), n, buf.buf.as<vmr::ONode>(), ctx->stream);
+  if (e == cudaSuccess) out = buf.buf.as<vmr::ONode>();
   return e;
 }
 
 // The octant copies of a motion tree; *bad_dev: the device flag that says whether
 // they may be used (null: there are none, and the traces walk the mnodes).
 cudaError_t octant_mnodes(vmr_ctx* ctx, const DevBuf& mnodes, const DevBuf& mboxes, uint32_t keys, uint32_t n,
-                          DevBuf& buf, int*& bad_dev) {
+                          vmr::OctantBuf& buf, int*& bad_dev) {
   bad_dev = nullptr;
   // an index plus the keys' offset stays below the kernels' markers
   if (n == 0 || (uint64_t)8 * keys * n >= 0xfffffffeull) return cudaSuccess;
   const size_t bytes = (size_t)8 * keys * n * sizeof(vmr::ONode);
-  cudaError_t e = buf.ensure(bytes + 16);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
-  if (e != cudaSuccess) return e;
-  bad_dev = reinterpret_cast<int*>(buf.as<char>() + bytes);
-  return (cudaError_t)vmr::launch_octant_mnodes(mnodes.as<MNode>(), mboxes.p, keys, n, buf.as<vmr::ONode>(), bad_dev,
-                                                ctx->stream);
+  bool got = false;
+  const cudaError_t e = octant_alloc(ctx, bytes + 16, buf, got);
+  if (e != cudaSuccess || !got) return e;
+  bad_dev = reinterpret_cast<int*>(buf.buf.as<char>() + bytes);
+  return (cudaError_t)vmr::launch_octant_mnodes(mnodes.as<MNode>(), mboxes.p, keys, n, buf.buf.as<vmr::ONode>(),
+                                                bad_dev, ctx->stream);
 }
 
 // Host accelerator -> device arrays (layout in device.h).  tris_ready: the
@@ -219,7 +241,8 @@ int upload_mesh(vmr_ctx* ctx, MeshRec& rec, bool tris_ready = false) {
   int bad = 0;
   if (bad_dev) VMR_CUDA(ctx, cudaMemcpyAsync(&bad, bad_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (bad_dev && !bad) d.onodes = rec.onodes.as<vmr::ONode>();
+  if (bad) rec.onodes.drop();
+  else if (bad_dev) d.onodes = rec.onodes.buf.as<vmr::ONode>();
   fill_xf(rec, d);
   rec.dmesh = d;
   for (int a = 0; a < 3; ++a) {
@@ -281,7 +304,8 @@ int refresh_top(vmr_ctx* ctx) {
   int bad = 0;
   if (bad_dev) VMR_CUDA(ctx, cudaMemcpyAsync(&bad, bad_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (bad_dev && !bad) d.onodes = t.onodes.as<vmr::ONode>();
+  if (bad) t.onodes.drop();
+  else if (bad_dev) d.onodes = t.onodes.buf.as<vmr::ONode>();
   d.geom_order = t.order.as<uint32_t>();
   d.meshes = t.meshes.as<DMesh>();
   d.n_geoms = (uint32_t)t.host.geom_order.size();

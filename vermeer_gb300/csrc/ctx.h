@@ -37,9 +37,31 @@ struct DevBuf {
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// A tree's octant copies, counted in *held, the sum over their context.
+struct OctantBuf {
+  DevBuf buf;
+  uint64_t* held = nullptr;
+  ~OctantBuf() { drop(); }
+  void drop() {
+    if (held) *held -= buf.bytes;
+    if (buf.p) cudaFree(buf.p);
+    buf.p = nullptr;
+    buf.bytes = 0;
+  }
+  cudaError_t ensure(size_t n, uint64_t* sum) {
+    if (n <= buf.bytes) return cudaSuccess;
+    drop();
+    held = sum;
+    const cudaError_t e = buf.ensure(n);
+    *held += buf.bytes;
+    return e;
+  }
+};
+
 struct MeshRec {
   HostMesh host;
-  DevBuf nodes, onodes, tris, mnodes, mboxes, mtris, elem;
+  OctantBuf onodes;
+  DevBuf nodes, tris, mnodes, mboxes, mtris, elem;
   DMesh dmesh{};
   float bounds6[6];
   // shading (render.cu): PolyMesh.Shader, shader index and normals per
@@ -128,7 +150,8 @@ struct GuideState {
 
 struct TopRec {
   HostTop host;
-  DevBuf nodes, onodes, mnodes, mboxes, order, meshes;
+  OctantBuf onodes;
+  DevBuf nodes, mnodes, mboxes, order, meshes;
   DTop dtop{};
   float bounds6[6] = {0, 0, 0, 0, 0, 0};  // union of the geoms' bounds (ray reordering)
   bool valid = false;
@@ -168,6 +191,8 @@ struct vmr_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evm = nullptr;  // start, after the sort, end
   // vmr_render's own start/end (its scene traces record ev0/ev1 themselves)
   cudaEvent_t rev0 = nullptr, rev1 = nullptr;
+  uint64_t octant_bytes = 0;      // the octant copies of meshes, top and flat, which count in it until they go
+  uint64_t device_bytes = 0;      // the device's memory (0: not asked yet)
   std::vector<std::unique_ptr<MeshRec>> meshes;
   TopRec top;
   vmr::FlatScene flat;
