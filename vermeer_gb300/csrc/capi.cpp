@@ -274,9 +274,15 @@ int refresh_top(vmr_ctx* ctx) {
   std::vector<DMesh> table(ctx->meshes.size());
   for (size_t i = 0; i < ctx->meshes.size(); ++i) table[i] = ctx->meshes[i]->dmesh;
   VMR_CUDA(ctx, upload(ctx, t.meshes, table));
+  // The tree stays as it is on the device unless t.host is a new one: a mesh's
+  // transform only changes the table and the flags below.
   DTop d{};
+  const bool tree = !t.on_device;
+  t.on_device = false;
   int* bad_dev = nullptr;
-  if (t.host.keys <= 1) {
+  if (!tree) {
+    d = t.dtop;
+  } else if (t.host.keys <= 1) {
     std::vector<GNode> g;
     if (!repack_nodes(t.host.nodes, (uint32_t)t.host.geom_order.size(), g))
       return fail(ctx, VMR_ERR_INVALID, "malformed top-level nodes");
@@ -300,7 +306,7 @@ int refresh_top(vmr_ctx* ctx) {
     d.n_nodes = d.n_mnodes;
     VMR_CUDA(ctx, octant_mnodes(ctx, t.mnodes, t.mboxes, d.keys, d.n_mnodes, t.onodes, bad_dev));
   }
-  VMR_CUDA(ctx, upload(ctx, t.order, t.host.geom_order));
+  if (tree) VMR_CUDA(ctx, upload(ctx, t.order, t.host.geom_order));
   int bad = 0;
   if (bad_dev) VMR_CUDA(ctx, cudaMemcpyAsync(&bad, bad_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VMR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -328,6 +334,7 @@ int refresh_top(vmr_ctx* ctx) {
   }
   t.dtop = d;
   t.valid = !t.host.geom_order.empty();
+  t.on_device = true;
   return VMR_OK;
 }
 
@@ -879,6 +886,7 @@ int vmr_scene_build(vmr_ctx* ctx, const uint32_t* geoms, uint32_t n) {
   HostTop top;
   if (!vmr::build_top_level(ms, ids, top, why)) return fail(ctx, VMR_ERR_INVALID, why);
   ctx->top.host = std::move(top);
+  ctx->top.on_device = false;
   return refresh_top(ctx);
 }
 
@@ -1027,6 +1035,7 @@ int vmr_scene_upload(vmr_ctx* ctx, const vmr_qbvh_node* nodes, uint32_t n_nodes,
     top.mboxes.assign(mboxes, mboxes + (size_t)keys * n_mnodes * 24);
   }
   ctx->top.host = std::move(top);
+  ctx->top.on_device = false;
   return refresh_top(ctx);
 }
 

@@ -155,6 +155,7 @@ struct TopRec {
   DTop dtop{};
   float bounds6[6] = {0, 0, 0, 0, 0, 0};  // union of the geoms' bounds (ray reordering)
   bool valid = false;
+  bool on_device = false;  // dtop's tree is host's (refresh_top)
 };
 
 // The camera the kernels see for a vmr_camera: m replaced by the matrix the
