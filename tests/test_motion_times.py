@@ -143,3 +143,47 @@ def test_motion_boxes_at_infinity(ctx, kind, keys, tris):
     ctx.scene_upload(t["geom_order"], mnodes=t["mnodes"],
                      mboxes=_reach_to_infinity(t["mboxes"].copy().reshape(keys, -1, 24), kind), keys=keys)
     _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
+
+
+@pytest.mark.parametrize("keys,tris,nodes", [(1, 780, 32), (1, 800, 33), (2, 303, 16), (2, 305, 17), (3, 241, 10),
+                                             (3, 237, 11)])
+@pytest.mark.parametrize("spoil", [False, True])
+def test_trees_around_the_size_whose_copies_the_host_makes(ctx, keys, tris, nodes, spoil):
+    """Up to 32 nodes times keys, and just above; spoil: a NaN plane in the last
+    node."""
+    from vermeer_gb300 import scenes
+    v, ip = scenes.triangle_soup(tris, 11, edge=0.06)
+    step = np.float32(0.05) * scenes.unit_sphere(5, v.shape[0], 3).astype(np.float32)
+    v = np.concatenate([v + np.float32(q) * step for q in range(keys)])
+    g = ctx.mesh_build(v, ip, keys=keys, motion_mode=1)
+    e = ctx.mesh_export(g)
+    assert len(e["nodes" if keys == 1 else "mnodes"]) == nodes
+    if spoil and keys == 1:
+        n = e["nodes"].copy()
+        n["boxes"].reshape(-1, 24)[-1, 13] = np.nan
+        g = ctx.mesh_upload(v, e["idxp"], e["accel_idx"], nodes=n, bounds=e["bounds"])
+    elif spoil:
+        b = e["mboxes"].copy().reshape(keys, -1, 24)
+        b[-1, -1, 13] = np.nan
+        g = ctx.mesh_upload(v, e["idxp"], e["accel_idx"], mnodes=e["mnodes"], mboxes=b, bounds=e["bounds"], keys=keys,
+                            motion_mode=1)
+    rays = _rays(4099, 59, (0.0, 1.0, 0.5))
+    r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_mesh(g, rays, shadow=shadow), OUT)
+    assert (r["prim"] >= 0).any()
+
+
+@pytest.mark.parametrize("n_geoms", [1, 2, 60, 80])
+@pytest.mark.parametrize("moving", [False, True])
+def test_top_levels_around_the_size_whose_copies_the_host_makes(ctx, n_geoms, moving):
+    from vermeer_gb300 import scenes
+    geoms = []
+    for k in range(n_geoms):
+        v, ip = scenes.triangle_soup(30, 200 + k, lo=0.01 * (k % 60), hi=0.01 * (k % 60) + 0.4, edge=0.08)
+        if moving and k % 4 == 0:
+            geoms.append(ctx.mesh_build(np.concatenate([v, v + np.float32(0.02)]), ip, keys=2, motion_mode=1))
+        else:
+            geoms.append(ctx.mesh_build(v, ip))
+    ctx.scene_build(geoms)
+    rays = _rays(4099, 61, (0.0, 1.0, 0.5))
+    r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_scene(rays, shadow=shadow), OUT + ("geom",))
+    assert (r["geom"] >= 0).any()

@@ -67,6 +67,55 @@ struct alignas(32) MNode {
 };
 static_assert(sizeof(MNode) == 32, "MNode must be 32 bytes");
 
+// Where octant o's copy holds child c of a node, and the child there.
+VMR_HD unsigned octant_slot(const uint32_t rank[2], unsigned c, unsigned o) {
+  return (rank[o >> 2] >> (8u * (o & 3u) + 2u * c)) & 3u;
+}
+// Static: a plane pair given in the wrong order is put in order and a NaN plane
+// takes the other's value, as the min and max of the products would; a child all
+// of whose planes are NaN is never hit.
+VMR_HD void octant_child(const GNode& N, unsigned c, unsigned o, ONode& r) {
+  const float inf = INFINITY;
+  const unsigned slot = octant_slot(N.rank, c, o);
+  const int at_near[3] = {0, 1, 4}, at_far[3] = {2, 3, 5};
+  float lo[3], hi[3];
+  int nans = 0;
+  for (int a = 0; a < 3; ++a) {
+    const float mn = N.box[c + 4 * a], mx = N.box[12 + c + 4 * a];
+    lo[a] = fminf(mn, mx);
+    hi[a] = fmaxf(mn, mx);
+    nans += lo[a] != lo[a] ? 1 : 0;
+  }
+  const bool absent = N.child[c] == kEmptyChild || nans == 3;
+  for (int a = 0; a < 3; ++a) {
+    const bool neg = (o >> a) & 1u;
+    // absent: near +inf and far -inf along D, whichever way D points
+    r.slot[slot][at_near[a]] = absent ? (neg ? -inf : inf) : (neg ? hi[a] : lo[a]);
+    r.slot[slot][at_far[a]] = absent ? (neg ? inf : -inf) : (neg ? lo[a] : hi[a]);
+  }
+  r.child[slot] = N.child[c];
+  r.pad[slot] = 0;
+}
+// Motion, one key's boxes (float[24], laid out as GNode::box); false when a
+// present child has a plane out of order, a NaN or an infinity (0 * inf at a key is
+// a NaN), where lerped near and far planes would not be the lerped box's: such a
+// tree keeps to its mnodes.
+VMR_HD bool octant_mchild(const MNode& N, const float* box, unsigned c, unsigned o, ONode& r) {
+  const unsigned slot = octant_slot(N.rank, c, o);
+  const int at_near[3] = {0, 1, 4}, at_far[3] = {2, 3, 5};
+  bool ok = true;
+  for (int a = 0; a < 3; ++a) {
+    const float mn = box[c + 4 * a], mx = box[12 + c + 4 * a];
+    const bool neg = (o >> a) & 1u;
+    ok = ok && mn <= mx && mn > -INFINITY && mx < INFINITY;
+    r.slot[slot][at_near[a]] = neg ? mx : mn;
+    r.slot[slot][at_far[a]] = neg ? mn : mx;
+  }
+  r.child[slot] = N.child[c];
+  r.pad[slot] = 0;
+  return ok || N.child[c] == kEmptyChild;
+}
+
 // The octant copies a context may hold, of a device with total bytes of memory:
 // a sixteenth, so a program that fills the device with geometry and workspaces of
 // its own still finds room for them.  (They are the faster walk at any mesh size:
@@ -226,9 +275,8 @@ int launch_ray_columns(const float* rows, uint64_t n, const RaySoA& out, void* s
 int launch_trace_scene(const DTop& top, const TraceLaunch& l);
 // out[8][n]: the octant copies of n nodes (traverse.cu).
 int launch_octant_nodes(const GNode* nodes, uint32_t n, ONode* out, void* stream);
-// out[8][keys][n] of n motion nodes; *bad is set when a box has its planes out
-// of order, a NaN or an infinity (0 * inf at a key is a NaN), where lerped near
-// and far planes would not be the lerped boxes' (such a mesh keeps to its mnodes).
+// out[8][keys][n] of n motion nodes; *bad is set when the tree keeps to its mnodes
+// (octant_mchild).
 int launch_octant_mnodes(const MNode* nodes, const void* mboxes, uint32_t keys, uint32_t n, ONode* out, int* bad,
                          void* stream);
 int device_sm_count();

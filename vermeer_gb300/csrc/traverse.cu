@@ -1073,67 +1073,21 @@ __device__ __forceinline__ void visit_octant_m(const ONode* p0, const ONode* p1,
       o.mask |= 1u << k;
 }
 
-// Octant copies of the nodes, a thread per child (a node of its own per thread left
-// small trees waiting for one thread's chain of loads and stores).
-//
-// Motion: the copies of every key; bad is set when a present child has a box whose
-// lerped near and far planes would not be the lerped box's.
+// Octant copies of the nodes (octant_child, octant_mchild), a thread per child: a
+// thread per copy left trees of few nodes waiting for its chain of loads and stores.
 __global__ void k_octant_mnodes(const MNode* __restrict__ nodes, const float* __restrict__ boxes, uint32_t keys,
                                 uint32_t n, ONode* __restrict__ out, int* bad) {
   const uint64_t per = (uint64_t)keys * n, total = per * 32;
   for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = (uint32_t)g & 3u, o = (uint32_t)(g / (4 * per));
     const uint64_t kn = (g >> 2) % per;
-    const MNode& N = nodes[kn % n];
-    const float* box = boxes + kn * 24;
-    const unsigned slot = (N.rank[o >> 2] >> (8u * (o & 3u) + 2u * c)) & 3u;
-    const int32_t child = N.child[c];
-    ONode& r = out[g >> 2];
-    const int at_near[3] = {0, 1, 4}, at_far[3] = {2, 3, 5};
-    for (int a = 0; a < 3; ++a) {
-      const float mn = box[c + 4 * a], mx = box[12 + c + 4 * a];
-      const bool neg = (o >> a) & 1u;
-      if (child != kEmptyChild && !(mn <= mx && isfinite(mn) && isfinite(mx))) *bad = 1;
-      r.slot[slot][at_near[a]] = neg ? mx : mn;
-      r.slot[slot][at_far[a]] = neg ? mn : mx;
-    }
-    r.child[slot] = child;
-    r.pad[slot] = 0;
+    if (!octant_mchild(nodes[kn % n], boxes + kn * 24, (unsigned)g & 3u, (unsigned)(g / (4 * per)), out[g >> 2])) *bad = 1;
   }
 }
 
-// Static: a plane pair given in the wrong order is put in order and a NaN plane
-// takes the other's value, as the min and max of the products would; a child all
-// of whose planes are NaN is never hit.
 __global__ void k_octant_nodes(const GNode* __restrict__ nodes, uint32_t n, ONode* __restrict__ out) {
   const uint64_t total = (uint64_t)n * 32;
-  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = (uint32_t)g & 3u, o = (uint32_t)(g / (4ull * n));
-    const GNode& N = nodes[(g >> 2) % n];
-    const unsigned slot = (N.rank[o >> 2] >> (8u * (o & 3u) + 2u * c)) & 3u;
-    const int32_t child = N.child[c];
-    float lo[3], hi[3];
-    int nans = 0;
-    for (int a = 0; a < 3; ++a) {
-      const float mn = N.box[c + 4 * a], mx = N.box[12 + c + 4 * a];
-      lo[a] = fminf(mn, mx);
-      hi[a] = fmaxf(mn, mx);
-      nans += isnan(lo[a]) ? 1 : 0;
-    }
-    const bool absent = child == kEmptyChild || nans == 3;
-    ONode& r = out[g >> 2];
-    const int at_near[3] = {0, 1, 4}, at_far[3] = {2, 3, 5};
-    for (int a = 0; a < 3; ++a) {
-      const bool neg = (o >> a) & 1u;
-      const float inf = __int_as_float(0x7f800000);
-      const float l = absent ? inf : lo[a], h = absent ? -inf : hi[a];
-      // absent: near +inf and far -inf along D, whichever way D points
-      r.slot[slot][at_near[a]] = absent ? (neg ? -inf : inf) : (neg ? h : l);
-      r.slot[slot][at_far[a]] = absent ? (neg ? inf : -inf) : (neg ? l : h);
-    }
-    r.child[slot] = child;
-    r.pad[slot] = 0;
-  }
+  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x)
+    octant_child(nodes[(g >> 2) % n], (unsigned)g & 3u, (unsigned)(g / (4ull * n)), out[g >> 2]);
 }
 
 // A traversal stack whose first SS entries per thread live in shared memory
