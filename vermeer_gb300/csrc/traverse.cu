@@ -1560,7 +1560,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
             tm = __fsub_rn(k, fk);
             omt = __fsub_rn(1.0f, tm);
             const int key = (int)fk, key2 = (int)ceilf(k);
-            if (!(k >= 0.0f) || key2 >= (int)m.keys) {
+            if (key < 0 || key2 >= (int)m.keys || k != k) {
               // out of the key range (the reference indexes out of bounds) or a
               // NaN time (its boxes are NaN, which no ray meets): miss
               store_end(hits, rid, r.tclosest, false);
@@ -1733,8 +1733,8 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
 // The key pair and lerp weight of a motion mesh at the ray's time
 // (builtin/geom/polymesh/trace.go:79-84); false outside the key range (the
 // reference would index out of bounds: a miss, as the mesh kernels treat it) and
-// for a NaN time, whose lerped boxes no ray meets.  Those tests are on k: the
-// integer of a NaN is 0, and slot_hit passes over a NaN plane.
+// for a NaN time, whose lerped boxes no ray meets (the integer of a NaN is 0, and
+// slot_hit passes over a NaN plane).
 __device__ __forceinline__ bool motion_keys(uint32_t keys, float time, float& tm, float& omt, int& key, int& key2) {
   const float k = __fmul_rn(time, (float)(keys - 1));
   const float fk = floorf(k);
@@ -1742,7 +1742,7 @@ __device__ __forceinline__ bool motion_keys(uint32_t keys, float time, float& tm
   omt = __fsub_rn(1.0f, tm);
   key = (int)fk;
   key2 = (int)ceilf(k);
-  return k >= 0.0f && key2 < (int)keys;
+  return !(key < 0 || key2 >= (int)keys || k != k);
 }
 
 // The walk is k_trace_mesh_ww's: octant copies of the current level's nodes,
