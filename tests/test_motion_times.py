@@ -98,6 +98,15 @@ def test_times_without_keys_miss_a_motion_mesh(ctx, keys, tris):
     rays = _rays(4099, 47, OUTSIDE + (np.nan,))
     r = _equal_to_kernel_0(ctx, lambda shadow: ctx.trace_mesh(g, rays, shadow=shadow), OUT)
     assert (r["prim"][::3] == -1).all() and ((r["prim"] >= 0).any() or tris == 1)
+    stats = []
+    try:
+        for k in (0, 13, 45):
+            ctx.set_tuning(kernel=k)
+            c = ctx.trace_mesh(g, rays, counters=True)["stats"]
+            stats.append([c[q] for q in ("node_visits", "leaf_visits", "tri_tests")])
+    finally:
+        ctx.set_tuning()
+    assert stats[1] == stats[0] and stats[2] == stats[0], stats
     # the same mesh under a top level that moves with it, and one that is still
     # beside it: nothing of such a scene is met
     w, iw = scenes.triangle_soup(40, 12, edge=0.2)

@@ -1562,7 +1562,8 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
             const int key = (int)fk, key2 = (int)ceilf(k);
             if (key < 0 || key2 >= (int)m.keys || k != k) {
               // out of the key range (the reference indexes out of bounds) or a
-              // NaN time (its boxes are NaN, which no ray meets): miss
+              // NaN time (the root's boxes are NaN, which no ray meets): miss
+              if (COUNT && k != k) cnt.nodes++;
               store_end(hits, rid, r.tclosest, false);
               alive = false;
             } else {
