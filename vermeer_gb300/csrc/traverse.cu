@@ -1550,7 +1550,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
           slab = slab_ray(r);
           obase = r.exact ? kNodesExact : !m.onodes ? kNodesPlain : r.oct * (MOTION ? m.keys : 1u) * m.n_nodes;
           sp = 0;
-          iter = 0;
+          iter = 1;
           alive = true;
           if (MOTION) {
             // k = Time*float32(keys-1); time = k-Floor(k); key = Floor(k),
@@ -1593,8 +1593,17 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
         }
         float T = 0.f;
         node = stk.get(--sp, T);
+        ++iter;
         if (ANY || !(r.tclosest < T)) return;
       }
+    };
+    // Every entry counts (node, leaf or culled): a tree whose nodes are reached more
+    // than once ends in a status, as in the other kernels.
+    auto capped = [&]() {
+      if (iter <= m.iter_cap) return;
+      status = kStatusIterationCap;
+      done = true;
+      walking = false;
     };
     if (alive) {
       // ---- node phase: one inner-node visit per step for every lane still
@@ -1610,12 +1619,6 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
           if (leafy != 0u) break;
         }
         if (!walking) continue;
-        if (++iter > m.iter_cap) {
-          status = kStatusIterationCap;
-          done = true;
-          walking = false;
-          continue;
-        }
         if (COUNT) cnt.nodes++;
         int next = 0;
         bool pushed;
@@ -1650,6 +1653,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
         }
         if (pushed) {
           node = next;
+          ++iter;
         } else if (status != kStatusOk) {
           done = true;
           walking = false;
@@ -1658,6 +1662,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
           pop();
         }
         walking = node >= 0;
+        capped();
       }
       // ---- leaf phase: lanes whose current entry is a leaf scan it, in the
       // order the reference pops it, then pop the next entry.
@@ -1676,6 +1681,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
           done = true;
         } else {
           pop();
+          capped();
           if (PF && !MOTION && node >= 0 && obase < kNodesPlain) prefetch_l1(m.onodes + (obase + (uint32_t)node));
         }
       }
@@ -1702,6 +1708,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : (MOTIO
           done = true;
         } else {
           pop();
+          capped();
         }
       }
     }
@@ -1777,7 +1784,10 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
   SlabRay slab{};
   int node = -1, sp = 0;
   uint64_t li = 0;  // the ray's position in rays
-  uint32_t iter = 0, miter = 0;  // visits left in the top level, in the mesh
+  // entries (nodes, leaves, culled ones) left in the top level, in the mesh; a step
+  // ends by looking at their signs: a tree whose nodes are reached more than once ends
+  // in a status, as in the other kernels
+  int iter = 0, miter = 0;
   bool alive = false, hit = false, more = true;
   bool need = false;  // the lane's next entry is to be found (next_entry)
   int status = kStatusOk;
@@ -1863,7 +1873,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
       return false;
     }
     geom = (int)g;
-    miter = M.iter_cap;
+    miter = (int)M.iter_cap - 1;  // its root
     node = 0;
     return true;
   };
@@ -1875,6 +1885,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
         while (sp > base) {
           float T = 0.f;
           const int e = stk.get(--sp, T);
+          --miter;
           if (ANY || !(r.tclosest < T)) {  // intersect.go:106
             node = e;
             return;
@@ -1906,6 +1917,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
       if (sp == 0) return;
       float T = 0.f;
       const int e = stk.get(--sp, T);
+      --iter;
       if (!ANY && r.tclosest < T) continue;
       node = e;
       if (node >= 0) return;
@@ -1935,7 +1947,8 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
           hit = false;
           node = -1;
           sp = 0;
-          iter = top.iter_cap;
+          iter = ray_path ? 0 : (int)top.iter_cap - 1;  // the root
+          miter = 0;
           geom = -1;
           leaf_left = 0;
           alive = true;
@@ -1970,51 +1983,51 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
         }
         if (!walking) continue;
         if (!need) {
-          if (geom < 0 ? iter-- == 0u : miter-- == 0u) {
-            status = kStatusIterationCap;
-          } else {
-            int next = 0;
-            bool pushed = false;
-            if (level != kLevelNodes) {
-              Slots o;
-              if (MOT && level == kLevelMotion) {
-                const float omt = __fsub_rn(1.0f, tm);
-                visit_octant_m(on + node, on + node + dkey, slab, tm, omt, r.tclosest, o);
-              } else {
-                visit_octant(on + node, slab, r.tclosest, o);
-              }
-              pushed = push_slots(stk, sp, o, next, status);
+          int next = 0;
+          bool pushed = false;
+          if (level != kLevelNodes) {
+            Slots o;
+            if (MOT && level == kLevelMotion) {
+              const float omt = __fsub_rn(1.0f, tm);
+              visit_octant_m(on + node, on + node + dkey, slab, tm, omt, r.tclosest, o);
             } else {
-              float4 b[6];
-              int4 ch;
-              unsigned rk;
-              const uint32_t keys = geom >= 0 ? top.meshes[geom].keys : top.keys;
-              if (MOT && keys > 1) {
-                float t, omt;
-                int key, key2;
-                motion_keys(keys, r.time, t, omt, key, key2);
-                const uint32_t nm = geom >= 0 ? top.meshes[geom].n_mnodes : top.n_mnodes;
-                const float4* bx = reinterpret_cast<const float4*>(geom >= 0 ? top.meshes[geom].mboxes : top.mboxes);
-                fetch_mnode(geom >= 0 ? top.meshes[geom].mnodes : top.mnodes, node, r.oct, bx + (size_t)key * nm * 6,
-                            bx + (size_t)key2 * nm * 6, t, omt, b, ch, rk);
-              } else {
-                uint4 meta;
-                ld_node((geom >= 0 ? top.meshes[geom].nodes : top.nodes) + node, b, ch, meta);
-                rk = (((r.oct & 4u) ? meta.z : meta.y) >> ((r.oct & 3u) * 8u)) & 0xffu;
-              }
-              int2 e[4];
-              const int np = visit_node(b, ch, rk, slab, r.exact, r.tclosest, e);
-              if (sp + np - 1 > kStackCapacity) {
-                status = kStatusStackOverflow;
-              } else if (np > 0) {
-                for (int k = 0; k + 1 < np; ++k) stk.set(sp++, e[k].x, __int_as_float(e[k].y));
-                next = e[np - 1].x;
-                pushed = true;
-              }
+              visit_octant(on + node, slab, r.tclosest, o);
             }
-            node = next;
-            need = !pushed;
-            if (pushed && node < 0 && geom < 0) {  // a top-level leaf
+            pushed = push_slots(stk, sp, o, next, status);
+          } else {
+            float4 b[6];
+            int4 ch;
+            unsigned rk;
+            const uint32_t keys = geom >= 0 ? top.meshes[geom].keys : top.keys;
+            if (MOT && keys > 1) {
+              float t, omt;
+              int key, key2;
+              motion_keys(keys, r.time, t, omt, key, key2);
+              const uint32_t nm = geom >= 0 ? top.meshes[geom].n_mnodes : top.n_mnodes;
+              const float4* bx = reinterpret_cast<const float4*>(geom >= 0 ? top.meshes[geom].mboxes : top.mboxes);
+              fetch_mnode(geom >= 0 ? top.meshes[geom].mnodes : top.mnodes, node, r.oct, bx + (size_t)key * nm * 6,
+                          bx + (size_t)key2 * nm * 6, t, omt, b, ch, rk);
+            } else {
+              uint4 meta;
+              ld_node((geom >= 0 ? top.meshes[geom].nodes : top.nodes) + node, b, ch, meta);
+              rk = (((r.oct & 4u) ? meta.z : meta.y) >> ((r.oct & 3u) * 8u)) & 0xffu;
+            }
+            int2 e[4];
+            const int np = visit_node(b, ch, rk, slab, r.exact, r.tclosest, e);
+            if (sp + np - 1 > kStackCapacity) {
+              status = kStatusStackOverflow;
+            } else if (np > 0) {
+              for (int k = 0; k + 1 < np; ++k) stk.set(sp++, e[k].x, __int_as_float(e[k].y));
+              next = e[np - 1].x;
+              pushed = true;
+            }
+          }
+          node = next;
+          need = !pushed;
+          if (pushed) {
+            if (geom < 0) --iter;
+            else --miter;
+            if (node < 0 && geom < 0) {  // a top-level leaf
               leaf_decode(node, leaf_next, leaf_left);
               need = true;
             }
@@ -2022,6 +2035,7 @@ __global__ void __launch_bounds__(128, MOT ? 4 : 6)
         }
         if (need && status == kStatusOk) next_entry();
         need = false;
+        if ((iter | miter) < 0) status = kStatusIterationCap;
         done = status != kStatusOk;
         walking = !done && node >= 0;
       }
