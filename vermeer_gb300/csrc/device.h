@@ -232,9 +232,11 @@ constexpr int kSortOctantBits = 4;
 constexpr int kSortBucketsMax = 2 * (6 << (3 * kSortMaxBits));  // the histogram, then its scan
 constexpr uint32_t sort_buckets(int bits) { return (6u << (3 * bits)) * (bits <= kSortOctantBits ? 4u : 1u); }
 // The width a tuning of 0 takes: 16^3 cells, or 8^3 for batches in which that
-// many buckets (98,304) would hold a few rays each and their scan costs more
-// than the finer cells give (300,007 rays: 488 against 495 us; 1,000,003: 460
-// against 456).
+// many buckets (98,304) hold a few rays each.  The two are within 2% of each other
+// from 65,536 to 1.5 million rays: 8^3 is 0.4 to 1.8% ahead for scenes up to 800,000
+// rays (300,007: 247 against 252 us; 1,000,003: 463 against 453; 3,000,000: 1,132
+// against 1,087), 16^3 0.5 to 1.3% for meshes from 300,000 (300,007: 619 against 615
+// us; 65,536: 348 against 351).
 constexpr int default_sort_bits(uint64_t n) { return n < 700000u ? 3 : 4; }
 constexpr uint64_t kSortMinRays = 1u << 16;  // smaller batches are traced unsorted
 

@@ -502,7 +502,10 @@ __global__ void __launch_bounds__(kPtBlock) k_pt_prep(PtBatch b, uint32_t d) {
 // 11.28 at 3 blocks, 11.10 at 4; with the queue 9.97 at 4 blocks, 10.20 at 3).
 // In a smaller batch a warp waits mostly on its own chain: warps alone at 3
 // blocks (80 registers), both directions' BSDF inline: 3,072 paths 576 us (590
-// with BIG), 16 jobs of 131,072 paths 6.32 ms (6.34).
+// with BIG), 16 jobs of 131,072 paths 6.32 ms (6.34).  In between BIG is ahead: by 0 to
+// 3% at 0.9 million paths, 2 to 5% at 2.8 to 3.7 million, as by 3 to 6% from 4.6 to 7.4
+// million (the 6 x 6 sphere grid and the room, depth 4 and 8), so the line could lie
+// lower.
 constexpr uint64_t kPtBigBatch = 1u << 22;
 template <bool BIG>
 __device__ __forceinline__ void phase_end() {

@@ -919,8 +919,9 @@ __global__ void k_jobs_scatter(const JobDesc* jobs, uint32_t n_jobs, uint64_t n,
 // count, lanes take base + their rank among the idle lanes), which keeps the
 // warp full until the ray pool runs dry.
 //
-// What bounds it: load latency and the L1 data pipe (about 75% of its
-// wavefronts; a visit costs one per lane and load instruction), then issue.
+// What bounds it: load latency (6.1 warps waiting on loads per issue) and the L1
+// data pipe (64% of its wavefronts; a visit costs one per lane and load
+// instruction), then issue (56% of cycles).
 // The octant copies exist to cut the work around those loads: push order and
 // near/far planes come with the node, two axes share an instruction, and a
 // step's pops follow its visit instead of taking steps of their own (of the
