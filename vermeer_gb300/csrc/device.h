@@ -275,7 +275,7 @@ int launch_ray_sort(const RaySoA& rays, uint64_t n, const float bounds[6], int b
 // n rays of 8 floats (16-byte aligned device memory) -> out's eight arrays.
 int launch_ray_columns(const float* rows, uint64_t n, const RaySoA& out, void* stream);
 int launch_trace_scene(const DTop& top, const TraceLaunch& l);
-// out[8][n]: the octant copies of n nodes (traverse.cu).
+// out[8][n]: the octant copies of n nodes (octant.cu).
 int launch_octant_nodes(const GNode* nodes, uint32_t n, ONode* out, void* stream);
 // out[8][keys][n] of n motion nodes; *bad is set when the tree keeps to its mnodes
 // (octant_mchild).
